@@ -1,0 +1,58 @@
+// The reference-layout hierarchy's coarse end on one thread-block cluster (cluster_tail.cuh).
+#include "cluster_tail.cuh"
+
+namespace ocub {
+
+using namespace ct;
+
+template <typename T>
+int cluster_tail_first(const std::vector<std::array<int, 3>> &dims) {
+  const int ranks = ct_max_ranks<CtPlain<T>>();
+  return ranks ? ct_first<CtPlain<T>>(dims, 1, kCtTopCells, ranks) : -1;
+}
+
+template <typename T>
+ocu_status launch_cluster_tail(const TailParams<T> &Q, bool ramp, cudaStream_t s) {
+  CtParams<CtPlain<T>> P;
+  std::memset(&P, 0, sizeof(P));
+  std::vector<std::array<int, 3>> dims;
+  for (int l = 0; l < Q.nlev; l++) dims.push_back({Q.lv[l].nx, Q.lv[l].ny, Q.lv[l].nz});
+  int ranks = 1;
+  const size_t bytes = ct_place(P, dims, 0, ct_max_ranks<CtPlain<T>>(), &ranks);
+  for (int l = 0; l < Q.nlev; l++) {
+    const TailLevel<T> &v = Q.lv[l];
+    P.lv[l].k = {v.rc, v.res};
+    P.lv[l].g = {v.u, v.b, v.xs, v.ys, v.hx, v.hy, v.hz};
+  }
+  P.nu1 = Q.nu1;
+  P.nu2 = Q.nu2;
+  P.post_first = Q.post_order == 1 ? 1 : 0;
+  P.coarse_iters = Q.coarse_iters;
+  if (Q.coarse_order == 2) {  // symmetric: an even number, at least four
+    if (P.coarse_iters % 2 == 1) P.coarse_iters++;
+    if (P.coarse_iters < 4) P.coarse_iters = 4;
+  }
+  P.coarse_flip = Q.coarse_order == 2 ? P.coarse_iters / 2 : P.coarse_iters;
+  P.host_coarse = Q.host_coarse;
+  P.x.cc = Q.cc;
+  P.x.unit = Q.cc.fx == 1 && Q.cc.fy == 1 && Q.cc.fz == 1;
+  P.x.bc = Q.lv[0].bc;
+  auto sign = [&](int f) {
+    const int t = P.x.bc.type[f];
+    return (T)(t == OCU_BC_NEUMANN ? 1 : t == OCU_BC_DIRICHELET ? -1 : 0);
+  };
+  auto periodic = [&](int f) { return P.x.bc.type[f] == OCU_BC_PERIODIC ? 1 : 0; };
+  P.sg = {sign(FX_NEG), sign(FX_POS), sign(FY_NEG), sign(FY_POS), sign(FZ_NEG), sign(FZ_POS),
+          periodic(FX_POS), periodic(FY_POS), periodic(FZ_POS)};
+  ct_schedule(P, ramp, ramp ? 0 : 1, Q.first_level == 0, 1LL << 62);
+  return ct_launch(P, ranks, bytes, s);
+}
+
+#define INST(T)                                                                     \
+  template int cluster_tail_first<T>(const std::vector<std::array<int, 3>> &);      \
+  template ocu_status launch_cluster_tail<T>(const TailParams<T> &, bool, cudaStream_t);
+INST(float)
+INST(double)
+#undef INST
+
+}  // namespace ocub

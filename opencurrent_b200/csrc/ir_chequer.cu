@@ -10,6 +10,7 @@
 #include <cstring>
 
 #include "chq_device.cuh"
+#include "cluster_tail.cuh"
 #include "mg_fused.h"
 
 namespace ocub {
@@ -190,11 +191,16 @@ ocu_status ChequerMG::init(const std::vector<std::array<int, 3>> &dims, const st
     total += 4 * (size_t)L.nx * L.ny * L.rz;
   }
   tail_s = tail_first(dims, tail_cells_setting());
-  size_t tail_bytes = 0;
-  for (size_t l = tail_s; l < dims.size(); l++) tail_bytes += level_smem(dims[l]);
+  if (!std::getenv("OCU_B200_CHQ_TAIL")) {
+    const int ranks = ct::ct_max_ranks<ct::CtChq>();
+    const int first = ranks ? ct::ct_first<ct::CtChq>(dims, 0, ct::kCtTopCells, ranks) : -1;
+    if (first >= 0) {
+      tail_s = first;
+      tail_ranks = ranks;
+    }
+  }
   OCU_TRY(check_cuda(cudaFuncSetAttribute(k_chq_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmemCap),
                      "cudaFuncSetAttribute (tail kernel)"));
-  (void)tail_bytes;
   OCU_TRY(check_cuda(cudaMalloc(&block, total * sizeof(float)), "cudaMalloc (FP32 refinement levels)"));
   OCU_TRY(check_cuda(cudaMemset(block, 0, total * sizeof(float)), "cudaMemset"));
   float *p = (float *)block;
@@ -262,7 +268,36 @@ ocu_status ChequerMG::prolong_from(int l, cudaStream_t s, int mode, double *x, c
   return check_launch("k_chq_prolong");
 }
 
-ocu_status ChequerMG::tail(bool fmg, int nu1, int nu2, int citers, cudaStream_t s) {
+ocu_status ChequerMG::tail_cluster(bool fmg, int more, int nu1, int nu2, int citers, int ramp_iters, cudaStream_t s) {
+  ct::CtParams<ct::CtChq> P;
+  std::memset(&P, 0, sizeof(P));
+  std::vector<std::array<int, 3>> dims;
+  for (const ChqLevel &C : lv) dims.push_back({C.nx, C.ny, C.nz});
+  int ranks = 1;
+  const size_t bytes = ct::ct_place(P, dims, tail_s, tail_ranks, &ranks);
+  for (int l = tail_s; l < levels(); l++) {
+    const ChqLevel &C = lv[l];
+    P.lv[l - tail_s].k = make_k(C.h, fx, fy, fz, omega);
+    P.lv[l - tail_s].g = {C.u[0], C.u[1], C.b[0], C.b[1], C.rz};
+  }
+  P.nu1 = nu1;
+  P.nu2 = nu2;
+  P.coarse_iters = P.coarse_flip = citers;
+  P.sg = ct::boundary_signs<float>(bc);
+  const ChqBC b = make_bc(bc, fx, fy, fz);
+  P.x = {b.mxn, b.mxp, b.myn, b.myp, b.mzn, b.mzp};
+  P.ramp_iters = ramp_iters;
+  ct::ct_schedule(P, fmg, more, tail_s == 0, kChqTailCells);
+  return ct::ct_launch(P, ranks, bytes, s);
+}
+
+ocu_status ChequerMG::tail(bool fmg, int more, int nu1, int nu2, int citers, int ramp_iters, cudaStream_t s) {
+  if (tail_ranks > 0) return tail_cluster(fmg, more, nu1, nu2, citers, ramp_iters, s);
+  if (fmg && more > 0) {
+    OCU_TRY(tail(true, 0, nu1, nu2, citers, ramp_iters, s));
+    fmg = false;
+  }
+  for (int c = 1; c < more; c++) OCU_TRY(tail(false, 1, nu1, nu2, citers, ramp_iters, s));
   ChqTail T{};
   const int L = levels();
   T.nlev = L - tail_s;
@@ -307,13 +342,14 @@ ocu_status ChequerMG::tail(bool fmg, int nu1, int nu2, int citers, cudaStream_t 
 ocu_status ChequerMG::enqueue_fmg(int nu1, int nu2, int cycles, int coarse_iters, int ramp_iters, cudaStream_t s,
                                   double *x, const ocu_layout *Lx) {
   const int ts = tail_s;
-  if (ts == 0) {  // the whole hierarchy in the single-CTA tail
-    OCU_TRY(tail(true, nu1, nu2, coarse_iters, s));
-    for (int c = 1; c < cycles; c++) OCU_TRY(tail(false, nu1, nu2, coarse_iters, s));
+  if (ts == 0) {  // the whole hierarchy in the tail
+    // the ramp ends with level 0's first V-cycle where the level is small enough for one
+    const bool small = (long long)lv[0].nx * lv[0].ny * lv[0].nz <= kChqTailCells;
+    OCU_TRY(tail(true, tail_ranks == 0 || small ? cycles - 1 : cycles, nu1, nu2, coarse_iters, ramp_iters, s));
     return x ? enqueue_add_correction(x, *Lx, s) : OCU_OK;
   }
   for (int l = 0; l < ts; l++) OCU_TRY(restrict_to(l, s, true));
-  OCU_TRY(tail(true, nu1, nu2, coarse_iters, s));
+  OCU_TRY(tail(true, 0, nu1, nu2, coarse_iters, ramp_iters, s));
   for (int f = ts - 1; f >= 1; f--) {
     OCU_TRY(prolong_from(f + 1, s, CHQ_P_ASSIGN));
     OCU_TRY(relax(f, ramp_iters, false, s));
@@ -325,7 +361,7 @@ ocu_status ChequerMG::enqueue_fmg(int nu1, int nu2, int cycles, int coarse_iters
       OCU_TRY(relax(l, nu1, false, s));
       OCU_TRY(restrict_to(l, s));
     }
-    OCU_TRY(tail(false, nu1, nu2, coarse_iters, s));
+    OCU_TRY(tail(false, 1, nu1, nu2, coarse_iters, ramp_iters, s));
     for (int l = ts - 1; l >= 0; l--) {
       if (l == 0 && x && c == cycles - 1) return prolong_from(1, s, xmode, x, Lx);
       OCU_TRY(prolong_from(l + 1, s));

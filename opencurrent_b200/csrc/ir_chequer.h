@@ -69,9 +69,11 @@ class ChequerMG {
   ocu_status restrict_to(int l, cudaStream_t s, bool zero_u = false);
   // mode: CHQ_P_ADD / ASSIGN / X64 / X64V (chq_device.cuh); x, Lx for the X64 modes
   ocu_status prolong_from(int l, cudaStream_t s, int mode = 0, double *x = nullptr, const ocu_layout *Lx = nullptr);
-  // levels tail_s..L-1 in one single-CTA launch: FMG (fmg) or one V-cycle from tail_s
-  ocu_status tail(bool fmg, int nu1, int nu2, int citers, cudaStream_t s);
+  // levels tail_s..L-1 in one launch: FMG (fmg), then `more` V-cycles from tail_s
+  ocu_status tail(bool fmg, int more, int nu1, int nu2, int citers, int ramp_iters, cudaStream_t s);
+  ocu_status tail_cluster(bool fmg, int more, int nu1, int nu2, int citers, int ramp_iters, cudaStream_t s);
   int tail_s = 0;
+  int tail_ranks = 0;  // most CTAs of the tail's cluster; 0: the single-CTA tail
 };
 
 }  // namespace ocub

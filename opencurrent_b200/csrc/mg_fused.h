@@ -2,6 +2,9 @@
 // relaxation, single-CTA tail parameters) and the fused-kernel launchers.
 #pragma once
 
+#include <array>
+#include <vector>
+
 #include "bc_device.cuh"
 #include "ocu_internal.h"
 
@@ -257,8 +260,14 @@ ocu_status launch_fold_rows(const T *rows, long long nrows, bool is_max, void *s
                             cudaStream_t s);
 template <typename T>
 ocu_status launch_coarse_tail(const TailParams<T> &P, cudaStream_t s);
-// The same schedule for `members` grids at once, one CTA per member.
-// The tail over the CTAs of one cluster (2..8 CTAs; every tail level with fused ghost writes).
+// The coarse end on one thread-block cluster (cluster_tail.cuh): the finest level >= 1 it takes,
+// or -1 (no level fits, or the device has no such clusters), and the launch of one V-cycle from
+// lv[0], or of the FMG ramp up to and including lv[0]'s V-cycle (lv[0]'s u is then taken as zero).
+template <typename T>
+int cluster_tail_first(const std::vector<std::array<int, 3>> &dims);
+template <typename T>
+ocu_status launch_cluster_tail(const TailParams<T> &P, bool ramp, cudaStream_t s);
+// The single-CTA schedule for `members` grids at once, one CTA per member.
 template <typename T>
 ocu_status launch_coarse_tail_batch(const TailParams<T> &P, const TailBatch &tb, int members, cudaStream_t s);
 

@@ -383,12 +383,37 @@ ocu_status MGCore<T>::prolong(int coarse, int fine) {
 template <typename T>
 int MGCore<T>::tail_start() const {
   const int coarse = num_levels - 1;
+  const int c = cluster_start();
+  if (c >= 1) return c;
   if (!fused || tail_cells <= 0) return coarse;
   int s = coarse;
   while (s - 1 >= 1 && (long long)dim[s - 1][0] * dim[s - 1][1] * dim[s - 1][2] <= tail_cells &&
          coarse - (s - 1) + 1 <= kMaxTailLevels)
     s--;
   return s;
+}
+
+// First level of the cluster's part, or -1 where the per-level kernels and the single-CTA tail run.
+template <typename T>
+int MGCore<T>::cluster_start() const {
+  return cluster && fused && !store_residuals ? cluster_tail_first<T>(dim) : -1;
+}
+
+template <typename T>
+ocu_status MGCore<T>::launch_tail_cluster(int s, int nu1, int nu2, int coarse_iters, bool symmetric, bool ramp) {
+  TailParams<T> P;
+  std::vector<T *> uo(num_levels), bo(num_levels);
+  for (int l = 0; l < num_levels; l++) {
+    uo[l] = u0(l);
+    bo[l] = b0(l);
+  }
+  fill_tail_params(P, s, nu1, nu2, coarse_iters, symmetric, uo.data(), bo.data());
+  return launch_cluster_tail<T>(P, ramp, stream);
+}
+
+template <typename T>
+ocu_status MGCore<T>::ramp_tail(int s, int nu1, int nu2, int coarse_iters, bool symmetric) {
+  return launch_tail_cluster(s, nu1, nu2, coarse_iters, symmetric, true);
 }
 
 // Tail schedule parameters for levels s..L-1 on the given level origins.
@@ -436,6 +461,8 @@ void MGCore<T>::fill_tail_params(TailParams<T> &P, int s, int nu1, int nu2, int 
 template <typename T>
 ocu_status MGCore<T>::cycle_tail(int s, int nu1, int nu2, int coarse_iters, bool symmetric) {
   const int coarse = num_levels - 1;
+  const int cs = cluster_start();
+  if (cs >= 1 && s >= cs) return launch_tail_cluster(s, nu1, nu2, coarse_iters, symmetric, false);
   if (s >= coarse) return relax(coarse, coarse_iters, symmetric ? RO_SYMMETRIC : RO_RED_BLACK);
   for (int l = s; l <= coarse; l++)
     if (!emit_ok(l) && l != coarse) {
@@ -589,10 +616,15 @@ ocu_status MGSolver::do_fmg_graph(double tolerance, int max_iter, double *rl2, d
     return OCU_OK;
   }
   OCU_TRY(run_segment(c, SEG_RAMP, [&]() -> ocu_status {
-    for (int level = 0; level < num_levels - 1; level++) {
+    const bool rt = c->ramp_in_tail();
+    for (int level = 0; level < (rt ? ts : num_levels - 1); level++) {
       OCU_TRY(c->clear_and_restrict(level, false, false));
     }
-    for (int f = num_levels - 1; f >= 1; f--) {
+    if (rt) {
+      OCU_TRY(c->ramp_tail(ts, prm.nu1, prm.nu2, coarse_iters(), prm.make_symmetric_operator != 0));
+      OCU_TRY(c->prolong(ts, ts - 1));
+    }
+    for (int f = rt ? ts - 1 : num_levels - 1; f >= 1; f--) {
       const int s = ts > f ? ts : f;
       OCU_TRY(enq_down(c, f, s));
       OCU_TRY(enq_tail_up(c, s, f));
@@ -995,6 +1027,7 @@ ocu_status MGSolver::apply_knobs() {
   cf.fused = cd.fused = prm.unfused == 0;
   cf.store_residuals = cd.store_residuals = prm.store_residual_grids != 0;
   cf.tail_cells = cd.tail_cells = tc;
+  cf.cluster = cd.cluster = prm.tail_cells == 0;
   cf.sweep_cells = cd.sweep_cells = prm.sweep_cells <= 0 ? kDefaultSweepCells : prm.sweep_cells;
   if (cf.sweep_cells > 0 && cf.num_levels > 0) OCU_TRY(cf.ensure_sweep_buffers());
   if (cd.sweep_cells > 0 && cd.num_levels > 0) OCU_TRY(cd.ensure_sweep_buffers());

@@ -51,6 +51,10 @@ struct CoreOps {
   // levels tail_start()..L-1 of a V-cycle in one launch
   virtual int tail_start() const = 0;
   virtual ocu_status cycle_tail(int s, int nu1, int nu2, int coarse_iters, bool symmetric) = 0;
+  // whether the tail also runs the FMG ramp: everything from the right-hand side of level s (u(s)
+  // zero) to the end of level s's ramp V-cycle, in one launch
+  virtual bool ramp_in_tail() const { return false; }
+  virtual ocu_status ramp_tail(int, int, int, int, bool) { return OCU_ERR_UNSUPPORTED; }
   // hierarchies spread over several streams: make the solver's stream wait for all of them
   // (join), and all of them wait for the solver's stream (fork: at the start of a stream capture,
   // so that their work joins the captured graph)
@@ -82,6 +86,7 @@ struct MGCore : CoreOps {
   bool fused = true;              // fused kernels (ghost writes, residual+restrict, tail)
   bool store_residuals = false;   // keep r_grid filled (reference kernels) for read_r
   int tail_cells = kDefaultTailCells;    // levels with at most this many cells run in the tail kernel
+  bool cluster = false;           // the levels that fit one thread-block cluster run there (tail_cells unused)
   int sweep_cells = kDefaultSweepCells;  // levels with at least this many cells use the two-colour pass
   // two-colour pass: per level a second u buffer (ping-pong) and the TMA maps of u, u2 and b
   std::vector<ocu_grid *> grids_u2;
@@ -99,6 +104,10 @@ struct MGCore : CoreOps {
   ocu_status clear_and_restrict(int fine, bool want_l2, bool want_linf) override;
   ocu_status finish_norms(int fine, double *l2, double *linf) override;
   int tail_start() const override;
+  int cluster_start() const;
+  bool ramp_in_tail() const override { return cluster_start() >= 1; }
+  ocu_status ramp_tail(int s, int nu1, int nu2, int coarse_iters, bool symmetric) override;
+  ocu_status launch_tail_cluster(int s, int nu1, int nu2, int coarse_iters, bool symmetric, bool ramp);
   ocu_status cycle_tail(int s, int nu1, int nu2, int coarse_iters, bool symmetric) override;
   void fill_tail_params(TailParams<T> &P, int s, int nu1, int nu2, int coarse_iters, bool symmetric,
                         T *const *u_origin, T *const *b_origin) const;
