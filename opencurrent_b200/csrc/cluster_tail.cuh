@@ -98,6 +98,7 @@ struct CtPlain {
     ct::hold(c.rc.omega), ct::hold(c.rc.hsq), ct::hold(c.rc.ld);
     ct::hold(c.rc.fx), ct::hold(c.rc.fy), ct::hold(c.rc.fz);
   }
+  static __device__ __forceinline__ void hold(Extra &x) { ct::hold(x.cc.omega), ct::hold(x.cc.ld), ct::hold(x.cc.h), ct::hold(x.unit); }
   // per-cell constant of the update: the diagonal
   static __device__ __forceinline__ T diag(int i, int j, int k, int nx, int ny, int nz, const Coef &c) {
     return relax_dg<T>(i, j, k, nx, ny, nz, c.rc, nullptr);
@@ -171,6 +172,7 @@ struct CtChq {
   }
   static constexpr bool kCornerFromPlus = false;
   static __device__ __forceinline__ float reciprocal(float) { return 0.f; }  // nothing is divided
+  static __device__ __forceinline__ void hold(Extra &) {}
   static __device__ __forceinline__ float update(float u, float b, float sx, float sy, float sz, float w, float,
                                                  const Coef &k, const Extra &, bool) {
     const float t = __fmaf_rn(k.fz, sz, __fmaf_rn(k.fy, sy, __fmaf_rn(k.fx, sx, -k.hsq * b)));
@@ -266,19 +268,34 @@ __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// A level's record in registers.  The records are indexed at run time, and read field by field
+// where they are used each read of the parameter bank is waited for on its own: here all are
+// asked for at once (a prolongation phase on an 8^3 level 2780 -> 2170 cycles, the clearing of a coarse
+// level 840 -> 690; 64^3 FP32 solve 470 -> 461 us).
+struct LevelRegs {
+  int nx, ny, nz, M, per, nact, ou, us, ob, bs;
+  FDiv fM, fY;
+};
 template <class Op>
-__device__ __forceinline__ int planes_of(const CtLevel<Op> &L, int r) {
+__device__ __forceinline__ LevelRegs level_regs(const CtLevel<Op> &R) {
+  LevelRegs L{R.nx, R.ny, R.nz, R.M, R.per, R.nact, R.ou, R.us, R.ob, R.bs, R.fM, R.fY};
+  asm volatile("" : "+r"(L.nx), "+r"(L.ny), "+r"(L.nz), "+r"(L.M), "+r"(L.per), "+r"(L.nact), "+r"(L.ou), "+r"(L.us),
+               "+r"(L.ob), "+r"(L.bs), "+r"(L.fM.d), "+r"(L.fM.sh), "+r"(L.fM.m), "+r"(L.fM.l), "+r"(L.fY.d),
+               "+r"(L.fY.sh), "+r"(L.fY.m), "+r"(L.fY.l));
+  return L;
+}
+template <class Lv>
+__device__ __forceinline__ int planes_of(const Lv &L, int r) {
   return max(0, min(L.per, L.nx - r * L.per));
 }
 // Barrier after a phase of a level.  A level that rank 0 holds alone is worked on by as many of
 // its warps as the level has pairs for (level_threads), on a named barrier of its own; the other
 // warps and ranks go on to the next visit that concerns them.
-template <class Op, int NT>
-__device__ __forceinline__ int level_threads(const CtLevel<Op> &L) {
+template <int NT, class Lv>
+__device__ __forceinline__ int level_threads(const Lv &L) {
   return L.nact > 1 ? NT : min(NT, (L.nx * L.ny * L.M + 31) & ~31);
 }
-template <class Op>
-__device__ __forceinline__ void level_barrier(const CtLevel<Op> &L, int l, int threads) {
+__device__ __forceinline__ void level_barrier(const LevelRegs &L, int l, int threads) {
   if (L.nact > 1) cluster_barrier();
   else if (threads == 32) __syncwarp();
   else asm volatile("bar.sync %0, %1;" ::"r"(l + 1), "r"(threads) : "memory");
@@ -297,7 +314,7 @@ struct Pair {
 };
 
 template <class Op>
-__device__ __forceinline__ Pair make_pair_at(const CtLevel<Op> &L, const BoundarySigns<typename Op::T> &sg,
+__device__ __forceinline__ Pair make_pair_at(const LevelRegs &L, const BoundarySigns<typename Op::T> &sg,
                                              unsigned ubase, int rank, int nl, int q) {
   constexpr int E = (int)sizeof(typename Op::T);
   Pair p;
@@ -326,10 +343,10 @@ __device__ __forceinline__ Pair make_pair_at(const CtLevel<Op> &L, const Boundar
 }
 
 template <class Op>
-__device__ __forceinline__ typename Op::T cell_constant(const CtParams<Op> &P, const CtLevel<Op> &L, int i, int j, int k,
-                                                        bool host) {
+__device__ __forceinline__ typename Op::T cell_constant(const CtParams<Op> &P, const LevelRegs &L,
+                                                        const typename Op::Coef &K, int i, int j, int k, bool host) {
   if constexpr (Op::kHostCoarse) {
-    return host ? Op::host_diag(i, j, k, L.nx, L.ny, L.nz, P.x.cc) : Op::diag(i, j, k, L.nx, L.ny, L.nz, L.k);
+    return host ? Op::host_diag(i, j, k, L.nx, L.ny, L.nz, P.x.cc) : Op::diag(i, j, k, L.nx, L.ny, L.nz, K);
   } else {
     float mod = 0.f;
     if (i == 0) mod += P.x.mxn;
@@ -338,22 +355,22 @@ __device__ __forceinline__ typename Op::T cell_constant(const CtParams<Op> &P, c
     if (j == L.ny - 1) mod += P.x.myp;
     if (k == 0) mod += P.x.mzn;
     if (k == L.nz - 1) mod += P.x.mzp;
-    return mod == 0.f ? 0.f : L.k.omega / (L.k.ld + mod);
+    return mod == 0.f ? 0.f : K.omega / (K.ld + mod);
   }
 }
 
 // Red-black sweeps of a slab of at most R * NT pairs, everything a sweep needs held in registers:
 // per cell the byte addresses of its five outer neighbours (across a face its own, with the
-// face's sign), value, right-hand side and update constant.  A phase of one warp is bound by the
-// number of its instructions: with neighbours selected by flags instead, and the pair's cell of
-// the sweep's colour by selects, it took 800 cycles on a 4^3 level, and 1230 with the loads inside
-// branches.
+// face's sign), value, right-hand side and update constant.  A sweep of one warp on a 4^3 level takes
+// 470-570 cycles; with neighbours selected by flags, and the pair's cell of the sweep's colour by
+// selects, 720, and 1150 with the loads inside branches.  (One loop for both colours, the registers
+// turned over by XOR between sweeps: 640.)
 // SIGNED: some face is neither Neumann nor periodic, so that a mirrored value carries a sign.
 template <class Op, int NT, int R, bool SIGNED>
-__device__ __forceinline__ void sweep_slab(const CtParams<Op> &P, const CtLevel<Op> &L, int l, int nthreads, char *U,
+__device__ __forceinline__ void sweep_slab(const CtParams<Op> &P, const LevelRegs &L, int l, int nthreads, char *U,
                                            const char *B, int rank, int nl, int n, int iters,
                                            int first, int flip, bool host, const typename Op::Coef &K,
-                                           const BoundarySigns<typename Op::T> &sg) {
+                                           const typename Op::Extra &X, const BoundarySigns<typename Op::T> &sg) {
   using T = typename Op::T;
   constexpr int E = (int)sizeof(T);
   const int us = L.us * E, bs = L.bs * E;
@@ -379,7 +396,7 @@ __device__ __forceinline__ void sweep_slab(const CtParams<Op> &P, const CtLevel<
       const int mine = c * us, other = (1 - c) * us;
       v[r][c] = *reinterpret_cast<const T *>(U + mine + p.id);
       b[r][c] = *reinterpret_cast<const T *>(B + c * bs + p.bid);
-      d[r][c] = cell_constant<Op>(P, L, p.i, p.j, 2 * p.m + odd, host);
+      d[r][c] = cell_constant<Op>(P, L, K, p.i, p.j, 2 * p.m + odd, host);
       rd[r][c] = Op::reciprocal(d[r][c]);
       xm[r][c] = p.xm + ((p.self & 1) ? mine : other);
       xp[r][c] = p.xp + ((p.self & 2) ? mine : other);
@@ -404,7 +421,7 @@ __device__ __forceinline__ void sweep_slab(const CtParams<Op> &P, const CtLevel<
             const T sx = SIGNED ? sxm[r] * ax + sxp[r] * bx : ax + bx;
             const T sy = SIGNED ? sym[r] * ay + syp[r] * by : ay + by;
             const T sz_ = (SIGNED ? sz[r][c] * az : az) + v[r][1 - c];
-            const T nv = Op::update(v[r][c], b[r][c], sx, sy, sz_, d[r][c], rd[r][c], K, P.x, host);
+            const T nv = Op::update(v[r][c], b[r][c], sx, sy, sz_, d[r][c], rd[r][c], K, X, host);
             v[r][c] = nv;
             *reinterpret_cast<T *>(U + c * us + own[r]) = nv;
             st_cl_if(left[r], c * us, nv);
@@ -424,16 +441,17 @@ template <class Op, int NT>
 __device__ __forceinline__ void visit_level(const CtParams<Op> &P, int what, int l, typename Op::T *sm, int rank) {
   using T = typename Op::T;
   constexpr int E = (int)sizeof(T);
-  const CtLevel<Op> &L = P.lv[l];
-  const CtLevel<Op> &Cl = P.lv[min(l + 1, P.nlev - 1)];
-  const int nthreads = level_threads<Op, NT>(L);
+  const CtLevel<Op> &coarser = P.lv[min(l + 1, P.nlev - 1)];
+  const LevelRegs L = level_regs(P.lv[l]);
+  const int nthreads = level_threads<NT>(L);
   const int nl = planes_of(L, rank), n = nl * L.ny * L.M;
-  const bool split_level = L.nact > 1, split_coarse = split_level && Cl.nact > 1;
+  const bool split_level = L.nact > 1, split_coarse = split_level && coarser.nact > 1;
   if ((what & CT_PROLONG) && !split_coarse) {
     level_barrier(L, l, nthreads);  // the coarser level is done
     if (split_level && rank != 0 && nl > 0) {
       // the planes of rank 0's level that this rank's cells read (halo planes included), into the
       // same place here: read one by one from every rank they cost 8000 cycles on rank 0's memory
+      const LevelRegs Cl = level_regs(coarser);
       const int S = Cl.ny * Cl.M, lo = ((rank * L.per) >> 1) * S, cnt = (((nl + 1) >> 1) + 2) * S;
       for (int q = threadIdx.x; q < 2 * cnt; q += NT) {
         const int e = Cl.ou + lo + (q < cnt ? q : q - cnt + Cl.us);
@@ -453,13 +471,15 @@ __device__ __forceinline__ void visit_level(const CtParams<Op> &P, int what, int
   const int flip = kind == CT_SWEEPS_COARSEST ? P.coarse_flip : iters;
   const int first = kind == CT_SWEEPS_POST ? P.post_first : 0;
   const int most = L.per * L.ny * L.M;  // pairs of the largest slab: the same choice on every rank
-  const int stride = Cl.per * Cl.ny * Cl.nz;  // residual scratch: elements per child
-  typename Op::Coef K = L.k;
+  typename Op::Coef K = P.lv[l].k;
+  typename Op::Extra X = P.x;
+  Op::hold(X);
   BoundarySigns<T> sg = P.sg;
   Op::hold(K);
   hold(sg.xn), hold(sg.xp), hold(sg.yn), hold(sg.yp), hold(sg.zn), hold(sg.zp);
   auto at = [](const char *base, int off) { return *reinterpret_cast<const T *>(base + off); };
   if (what & CT_PROLONG) {
+      const LevelRegs Cl = level_regs(coarser);
       for (int q = threadIdx.x; q < n; q += NT) {
         const Pair p = make_pair_at<Op>(L, sg, ubase, rank, nl, q);
         const int c0 = (p.i + p.j) & 1;
@@ -520,9 +540,9 @@ __device__ __forceinline__ void visit_level(const CtParams<Op> &P, int what, int
     const bool plus = (sg.px || (sg.xn == (T)1 && sg.xp == (T)1)) && (sg.py || (sg.yn == (T)1 && sg.yp == (T)1)) &&
                       (sg.pz || (sg.zn == (T)1 && sg.zp == (T)1));
     if (plus && most <= NT)
-      sweep_slab<Op, NT, 1, false>(P, L, l, nthreads, U, B, rank, nl, n, iters, first, flip, host, K, sg);
+      sweep_slab<Op, NT, 1, false>(P, L, l, nthreads, U, B, rank, nl, n, iters, first, flip, host, K, X, sg);
     else if (most <= NT)
-      sweep_slab<Op, NT, 1, true>(P, L, l, nthreads, U, B, rank, nl, n, iters, first, flip, host, K, sg);
+      sweep_slab<Op, NT, 1, true>(P, L, l, nthreads, U, B, rank, nl, n, iters, first, flip, host, K, X, sg);
     else {  // pairs worked out again in every phase
       for (int ph = 0; ph < 2 * iters; ph++) {
         const int color = (ph & 1) ^ (ph < 2 * flip ? first : 1 - first);
@@ -535,8 +555,8 @@ __device__ __forceinline__ void visit_level(const CtParams<Op> &P, int what, int
           const T sx = ((p.self & 1) ? sg.xn * u : lxm) + ((p.self & 2) ? sg.xp * u : lxp);
           const T sy = ((p.self & 4) ? sg.yn * u : lym) + ((p.self & 8) ? sg.yp * u : lyp);
           const T zv = (p.self & (odd ? 32 : 16)) ? (odd ? sg.zp : sg.zn) * u : lz;
-          const T d = cell_constant<Op>(P, L, p.i, p.j, 2 * p.m + odd, host);
-          const T nv = Op::update(u, at(B, color * bs + p.bid), sx, sy, zv + at(O, p.id), d, Op::reciprocal(d), K, P.x, host);
+          const T d = cell_constant<Op>(P, L, K, p.i, p.j, 2 * p.m + odd, host);
+          const T nv = Op::update(u, at(B, color * bs + p.bid), sx, sy, zv + at(O, p.id), d, Op::reciprocal(d), K, X, host);
           *reinterpret_cast<T *>(U + color * us + p.id) = nv;
           st_cl_if(p.left, color * us, nv);
           st_cl_if(p.right, color * us, nv);
@@ -546,6 +566,8 @@ __device__ __forceinline__ void visit_level(const CtParams<Op> &P, int what, int
     }
   }
   if (!(what & CT_RESTRICT)) return;
+  const LevelRegs Cl = level_regs(coarser);
+  const int stride = Cl.per * Cl.ny * Cl.nz;  // residual scratch: elements per child
   {
       for (int q = threadIdx.x; q < n; q += NT) {
         const Pair p = make_pair_at<Op>(L, sg, ubase, rank, nl, q);
@@ -581,7 +603,7 @@ __device__ __forceinline__ void visit_level(const CtParams<Op> &P, int what, int
     else level_barrier(L, l, nthreads);
   }
   // the coarse owner adds up each cell's eight residuals and clears u (halos included)
-  const int cthreads = level_threads<Op, NT>(Cl);
+  const int cthreads = level_threads<NT>(Cl);
   if (Cl.nact == 1 && (rank != 0 || (int)threadIdx.x >= cthreads)) return;
   const int cl = planes_of(Cl, rank), cn = cl * Cl.ny * Cl.M, S = Cl.ny * Cl.M;
   const T *r = sm + P.orr;
@@ -618,7 +640,7 @@ __device__ __forceinline__ void run_schedule(const CtParams<Op> &P, typename Op:
     if (pc >= P.once && (left <= 0 || P.once == P.total)) break;
     const int step = P.prog[pc++], l = step >> 5;
     const CtLevel<Op> &L = P.lv[l];
-    if (L.nact == 1 && (rank != 0 || (int)threadIdx.x >= level_threads<Op, NT>(L))) continue;
+    if (L.nact == 1 && (rank != 0 || (int)threadIdx.x >= level_threads<NT>(L))) continue;
     visit_level<Op, NT>(P, step & 31, l, sm, rank);
   }
 }
