@@ -841,10 +841,13 @@ __global__ void __launch_bounds__(256) k_residual_restrict_fine(const T *__restr
 }
 
 // 256-wide fold of row values (grid1dops.cu:33-115), one launch: block b folds rows
-// [256b, 256b+256), the last block folds the block partials.  Writes the T result as double.
+// [256b, 256b+256), the last block folds the block partials.  Writes the T result as double, and
+// where `host` is given then copies the n norms at `norms` (the result among them) into that
+// pinned host memory, as k_readback does: a launch of its own cost 2.3 us a multigrid cycle.
 template <typename T>
 __global__ void __launch_bounds__(256) k_fold_rows(const T *__restrict__ rows, long long nrows, int is_max,
-                                                   T *partial, unsigned *counter, double *result) {
+                                                   T *partial, unsigned *counter, double *result,
+                                                   const volatile double *norms, double *host, int n) {
   pdl_entry();
   __shared__ T sh[256];
   __shared__ bool last;
@@ -885,6 +888,8 @@ __global__ void __launch_bounds__(256) k_fold_rows(const T *__restrict__ rows, l
   if (threadIdx.x == 0) {
     *result = (double)vp[0];
     *counter = 0;
+    for (int q = 0; q < n; q++) host[q] = norms + q == result ? (double)vp[0] : norms[q];
+    if (n > 0) __threadfence_system();
   }
 }
 
@@ -950,11 +955,12 @@ ocu_status launch_residual_restrict(const T *u, const T *b, const ocu_layout &Lf
 
 template <typename T>
 ocu_status launch_fold_rows(const T *rows, long long nrows, bool is_max, void *scratch, double *result,
-                            cudaStream_t s) {
+                            cudaStream_t s, const double *norms, double *host, int n) {
   const long long blocks = (nrows + 255) / 256;
   unsigned *counter = reinterpret_cast<unsigned *>(scratch);
   T *partial = reinterpret_cast<T *>(reinterpret_cast<char *>(scratch) + 64);
-  launch_pdl(k_fold_rows<T>, (unsigned)blocks, 256, 0, s, rows, nrows, is_max ? 1 : 0, partial, counter, result);
+  launch_pdl(k_fold_rows<T>, (unsigned)blocks, 256, 0, s, rows, nrows, is_max ? 1 : 0, partial, counter, result,
+             norms, host, host ? n : 0);
   return check_launch("k_fold_rows");
 }
 
@@ -1545,7 +1551,8 @@ INST_B(double)
   template ocu_status launch_residual_restrict<T>(const T *, const T *, const ocu_layout &, T *,                \
                                                   const ocu_layout &, double, double, double, double, T *, T *, \
                                                   cudaStream_t, T *, long long);                               \
-  template ocu_status launch_fold_rows<T>(const T *, long long, bool, void *, double *, cudaStream_t);          \
+  template ocu_status launch_fold_rows<T>(const T *, long long, bool, void *, double *, cudaStream_t,              \
+                                          const double *, double *, int);          \
   template ocu_status launch_coarse_tail<T>(const TailParams<T> &, cudaStream_t);                               \
   template ocu_status launch_coarse_tail_batch<T>(const TailParams<T> &, const TailBatch &, int, cudaStream_t);
 INST(float)

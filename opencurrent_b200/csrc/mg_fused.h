@@ -257,7 +257,7 @@ ocu_status launch_residual_restrict(const T *u, const T *b, const ocu_layout &Lf
                                     T *zero_u = nullptr, long long zero_n = 0);
 template <typename T>
 ocu_status launch_fold_rows(const T *rows, long long nrows, bool is_max, void *scratch, double *result,
-                            cudaStream_t s);
+                            cudaStream_t s, const double *norms = nullptr, double *host = nullptr, int n = 0);
 template <typename T>
 ocu_status launch_coarse_tail(const TailParams<T> &P, cudaStream_t s);
 // The coarse end on one thread-block cluster (cluster_tail.cuh): the finest level >= 1 it takes,

@@ -309,9 +309,7 @@ ocu_status MGCore<T>::enqueue_restrict_residuals(int fine, int coarse, bool want
       OCU_TRY(launch_residual_rows<T>(u0(fine), b0(fine), nullptr, nullptr, lay[fine], hf, fx, fy, fz, rows2, rowsinf,
                                       stream));
     }
-    const long long nrows = (long long)dim[fine][0] * dim[fine][1];
-    if (want_l2) OCU_TRY(launch_fold_rows<T>(rows2, nrows, false, red_scratch, d_norms, stream));
-    if (want_linf) OCU_TRY(launch_fold_rows<T>(rowsinf, nrows, true, red_scratch, d_norms + 1, stream));
+    return enqueue_norms(fine, rows2, rowsinf);
   }
   if (norms)
     OCU_TRY(launch_readback(d_norms, h_norms, 3, stream));
@@ -328,17 +326,22 @@ ocu_status MGCore<T>::clear_and_restrict(int fine, bool want_l2, bool want_linf)
     OCU_TRY(clear_level(coarse));
     return enqueue_restrict_residuals(fine, coarse, want_l2, want_linf);
   }
-  const bool norms = want_l2 || want_linf;
   T *rows2 = want_l2 ? (T *)rows : nullptr;
   T *rowsinf = want_linf ? (T *)rows + rows_stride : nullptr;
   OCU_TRY(launch_residual_restrict<T>(u0(fine), b0(fine), lay[fine], b0(coarse), lay[coarse], h[fine], fx, fy, fz,
                                       rows2, rowsinf, stream, static_cast<T *>(grids_u[coarse]->buf),
                                       lay[coarse].allocated));
+  return enqueue_norms(fine, rows2, rowsinf);
+}
+
+// Folds the row values that are asked for; the last fold also takes the norms and the timeout
+// word to pinned host memory (finish_norms waits).
+template <typename T>
+ocu_status MGCore<T>::enqueue_norms(int fine, const T *rows2, const T *rowsinf) {
   const long long nrows = (long long)dim[fine][0] * dim[fine][1];
-  if (want_l2) OCU_TRY(launch_fold_rows<T>(rows2, nrows, false, red_scratch, d_norms, stream));
-  if (want_linf) OCU_TRY(launch_fold_rows<T>(rowsinf, nrows, true, red_scratch, d_norms + 1, stream));
-  if (norms)
-    OCU_TRY(launch_readback(d_norms, h_norms, 3, stream));
+  if (rows2)
+    OCU_TRY(launch_fold_rows<T>(rows2, nrows, false, red_scratch, d_norms, stream, d_norms, rowsinf ? nullptr : h_norms, 3));
+  if (rowsinf) OCU_TRY(launch_fold_rows<T>(rowsinf, nrows, true, red_scratch, d_norms + 1, stream, d_norms, h_norms, 3));
   return OCU_OK;
 }
 
@@ -523,6 +526,9 @@ static double pick(int conv, double l2, double linf) {
 //   RAMP   restriction chain + the FMG cycles from the coarsest level up to level 1
 //   PRE0   pre-smooth at level 0, clear level 1, residual+restriction+norms (read back)
 //   REST0  the rest of a level-0 cycle (levels 1.. down, tail kernel, up to level 0)
+// What runs between two readbacks is one graph (the ramp with the first PRE0, a REST0 with the next
+// cycle's PRE0), so that the programmatic dependencies are not broken between them; a REST0 on its
+// own ends a run that stops at max_iter.
 //   FINAL  ghost fill of u0 after convergence
 // With CONVERGENCE_NONE nothing is read back, so a whole fixed-schedule FMG (the refinement
 // solver's inner solve) runs as a chain of graph launches without a host wait.
@@ -574,7 +580,7 @@ ocu_status MGSolver::run_segment(const void *core, int seg, F &&enqueue) {
   return OCU_OK;
 }
 
-enum { SEG_INIT = 0, SEG_RAMP = 8, SEG_PRE0 = 16, SEG_REST0 = 24, SEG_FINAL = 32 };
+enum { SEG_INIT = 0, SEG_PRE0 = 16, SEG_REST0 = 24, SEG_FINAL = 32, SEG_RAMP_PRE0 = 40, SEG_REST0_PRE0 = 48 };
 
 // levels [a, b) of a down-leg without norm checks
 ocu_status MGSolver::enq_down(CoreOps *c, int a, int b) {
@@ -602,6 +608,10 @@ ocu_status MGSolver::do_fmg_graph(double tolerance, int max_iter, double *rl2, d
   const int nv = (wl2 ? 1 : 0) + (wlinf ? 2 : 0);
   CoreOps *c = active();
   const int ts = c->tail_start();
+  auto pre0 = [&]() -> ocu_status {
+    OCU_TRY(c->relax(0, prm.nu1, RO_RED_BLACK));
+    return c->clear_and_restrict(0, wl2, wlinf);
+  };
   double orig_l2 = 0, orig_linf = 0;
   *rl2 = *rlinf = 0;
   OCU_TRY(run_segment(c, SEG_INIT + nv, [&]() -> ocu_status {
@@ -615,7 +625,7 @@ ocu_status MGSolver::do_fmg_graph(double tolerance, int max_iter, double *rl2, d
     stats.vcycles = 0;
     return OCU_OK;
   }
-  OCU_TRY(run_segment(c, SEG_RAMP, [&]() -> ocu_status {
+  OCU_TRY(run_segment(c, SEG_RAMP_PRE0 + nv, [&]() -> ocu_status {
     const bool rt = c->ramp_in_tail();
     for (int level = 0; level < (rt ? ts : num_levels - 1); level++) {
       OCU_TRY(c->clear_and_restrict(level, false, false));
@@ -630,15 +640,11 @@ ocu_status MGSolver::do_fmg_graph(double tolerance, int max_iter, double *rl2, d
       OCU_TRY(enq_tail_up(c, s, f));
       OCU_TRY(c->prolong(f, f - 1));
     }
-    return OCU_OK;
+    return pre0();
   }));
   int num_vcyc = 0;
   for (int i_cyc = 0; i_cyc < max_iter + 1; i_cyc++) {
     num_vcyc++;
-    OCU_TRY(run_segment(c, SEG_PRE0 + nv, [&]() -> ocu_status {
-      OCU_TRY(c->relax(0, prm.nu1, RO_RED_BLACK));
-      return c->clear_and_restrict(0, wl2, wlinf);
-    }));
     if (wl2 || wlinf) {
       OCU_TRY(c->finish_norms(0, wl2 ? rl2 : nullptr, wlinf ? rlinf : nullptr));
       stats.last_l2 = *rl2;
@@ -649,9 +655,11 @@ ocu_status MGSolver::do_fmg_graph(double tolerance, int max_iter, double *rl2, d
       stats.vcycles = num_vcyc;
       return OCU_OK;
     }
-    OCU_TRY(run_segment(c, SEG_REST0, [&]() -> ocu_status {
+    const bool more = i_cyc < max_iter;  // another cycle follows
+    OCU_TRY(run_segment(c, more ? SEG_REST0_PRE0 + nv : SEG_REST0, [&]() -> ocu_status {
       OCU_TRY(enq_down(c, 1, ts));
-      return enq_tail_up(c, ts, 0);
+      OCU_TRY(enq_tail_up(c, ts, 0));
+      return more ? pre0() : OCU_OK;
     }));
   }
   stats.vcycles = num_vcyc;
@@ -664,6 +672,10 @@ ocu_status MGSolver::do_vcycle_graph(double tolerance, int max_iter, double *rl2
   const int nv = (wl2 ? 1 : 0) + (wlinf ? 2 : 0);
   CoreOps *c = active();
   const int ts = c->tail_start();
+  auto pre0 = [&]() -> ocu_status {
+    OCU_TRY(c->relax(0, prm.nu1, RO_RED_BLACK));
+    return c->clear_and_restrict(0, wl2, wlinf);
+  };
   double orig_l2 = 0, orig_linf = 0;
   OCU_TRY(run_segment(c, SEG_INIT + nv, [&]() -> ocu_status {
     OCU_TRY(c->apply_bc(0));
@@ -676,18 +688,17 @@ ocu_status MGSolver::do_vcycle_graph(double tolerance, int max_iter, double *rl2
     return OCU_OK;
   }
   for (int i_cyc = 0; i_cyc < max_iter; i_cyc++) {
-    OCU_TRY(run_segment(c, SEG_PRE0 + nv, [&]() -> ocu_status {
-      OCU_TRY(c->relax(0, prm.nu1, RO_RED_BLACK));
-      return c->clear_and_restrict(0, wl2, wlinf);
-    }));
+    if (i_cyc == 0) OCU_TRY(run_segment(c, SEG_PRE0 + nv, pre0));
     if (wl2 || wlinf) OCU_TRY(c->finish_norms(0, wl2 ? rl2 : nullptr, wlinf ? rlinf : nullptr));
     if (pick(conv, *rl2, *rlinf) < tolerance) {
       OCU_TRY(run_segment(c, SEG_FINAL, [&]() -> ocu_status { return c->apply_bc(0); }));
       return OCU_OK;
     }
-    OCU_TRY(run_segment(c, SEG_REST0, [&]() -> ocu_status {
+    const bool more = i_cyc + 1 < max_iter;  // another cycle follows
+    OCU_TRY(run_segment(c, more ? SEG_REST0_PRE0 + nv : SEG_REST0, [&]() -> ocu_status {
       OCU_TRY(enq_down(c, 1, ts));
-      return enq_tail_up(c, ts, 0);
+      OCU_TRY(enq_tail_up(c, ts, 0));
+      return more ? pre0() : OCU_OK;
     }));
   }
   return OCU_ERR_NOT_CONVERGED;
@@ -862,11 +873,8 @@ enum { SEG_CHQ_FIRST = 0, SEG_CHQ_STEP = 1 };
 ocu_status MGSolver::ir_chequer_residual_tail() {
   const ocu_layout &L = cd.lay[0];
   double *rows2 = (double *)cd.rows, *rowsinf = (double *)cd.rows + cd.rows_stride;
-  const long long nrows = (long long)L.nx * L.ny;
   OCU_TRY(chq->enqueue_residual(cd.u0(0), cd.b0(0), L, cd.h[0], cd.fx, cd.fy, cd.fz, rows2, rowsinf, stream));
-  OCU_TRY(launch_fold_rows<double>(rows2, nrows, false, cd.red_scratch, cd.d_norms, stream));
-  OCU_TRY(launch_fold_rows<double>(rowsinf, nrows, true, cd.red_scratch, cd.d_norms + 1, stream));
-  return launch_readback(cd.d_norms, cd.h_norms, 3, stream);
+  return cd.enqueue_norms(0, rows2, rowsinf);
 }
 
 ocu_status MGSolver::ir_solve_chequer(double tolerance, int max_outer, double *rl2, double *rlinf) {
@@ -912,10 +920,7 @@ ocu_status MGSolver::ir_residual(double *l2, double *linf) {
   double *rows2 = (double *)cd.rows, *rowsinf = (double *)cd.rows + cd.rows_stride;
   OCU_TRY(launch_residual_rows<double>(cd.u0(0), cd.b0(0), nullptr, (float *)cf.b0(0), L, cd.h[0], cd.fx, cd.fy,
                                        cd.fz, rows2, rowsinf, stream));
-  const long long nrows = (long long)L.nx * L.ny;
-  OCU_TRY(launch_fold_rows<double>(rows2, nrows, false, cd.red_scratch, cd.d_norms, stream));
-  OCU_TRY(launch_fold_rows<double>(rowsinf, nrows, true, cd.red_scratch, cd.d_norms + 1, stream));
-  OCU_TRY(launch_readback(cd.d_norms, cd.h_norms, 3, stream));
+  OCU_TRY(cd.enqueue_norms(0, rows2, rowsinf));
   return cd.finish_norms(0, l2, linf);
 }
 

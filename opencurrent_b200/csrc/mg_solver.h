@@ -103,6 +103,7 @@ struct MGCore : CoreOps {
   ocu_status enqueue_restrict_residuals(int fine, int coarse, bool want_l2, bool want_linf) override;
   ocu_status clear_and_restrict(int fine, bool want_l2, bool want_linf) override;
   ocu_status finish_norms(int fine, double *l2, double *linf) override;
+  ocu_status enqueue_norms(int fine, const T *rows2, const T *rowsinf);
   int tail_start() const override;
   int cluster_start() const;
   bool ramp_in_tail() const override { return cluster_start() >= 1; }
