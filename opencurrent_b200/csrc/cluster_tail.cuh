@@ -359,80 +359,93 @@ __device__ __forceinline__ typename Op::T cell_constant(const CtParams<Op> &P, c
   }
 }
 
-// Red-black sweeps of a slab of at most R * NT pairs, everything a sweep needs held in registers:
-// per cell the byte addresses of its five outer neighbours (across a face its own, with the
-// face's sign), value, right-hand side and update constant.  A sweep of one warp on a 4^3 level takes
-// 470-570 cycles; with neighbours selected by flags, and the pair's cell of the sweep's colour by
-// selects, 720, and 1150 with the loads inside branches.  (One loop for both colours, the registers
-// turned over by XOR between sweeps: 640.)
-// SIGNED: some face is neither Neumann nor periodic, so that a mirrored value carries a sign.
-template <class Op, int NT, int R, bool SIGNED>
+// Exchanges a register's two colours: m is the XOR of the values for one and the other.
+__device__ __forceinline__ int flip_bits(float a, float b) { return __float_as_int(a) ^ __float_as_int(b); }
+__device__ __forceinline__ long long flip_bits(double a, double b) { return __double_as_longlong(a) ^ __double_as_longlong(b); }
+__device__ __forceinline__ void flip_value(float &v, int m) { v = __int_as_float(__float_as_int(v) ^ m); }
+__device__ __forceinline__ void flip_value(double &v, long long m) { v = __longlong_as_double(__double_as_longlong(v) ^ m); }
+
+// Red-black sweeps of a slab of at most NT pairs, everything a sweep needs held in registers: of the
+// cell of the sweep's colour the byte addresses of its five outer neighbours (across a face its
+// own, with the face's sign), its value, right-hand side and update constant, each turned into
+// the other cell's by one XOR between sweeps.  A sweep costs the instructions of its busiest warp, 4
+// to 5 cycles each: on a 4^3 level 520 (FP64) to 600 cycles, 580 to 680 with both colours' code and
+// both arithmetics in the loop, 720 with the neighbours and the pair's cell chosen by flags, 1150
+// with the loads inside branches; loads, division and remote stores are 130 of them.  One pair a
+// thread: two or four in registers, or 1024 threads of 64 registers, were slower (set-up, spills).
+// HOST: the coarsest level's arithmetic; SIGNED: some face is neither Neumann nor periodic, so that
+// a mirrored value carries a sign.
+template <class Op, int NT, bool HOST, bool SIGNED>
 __device__ __forceinline__ void sweep_slab(const CtParams<Op> &P, const LevelRegs &L, int l, int nthreads, char *U,
-                                           const char *B, int rank, int nl, int n, int iters,
-                                           int first, int flip, bool host, const typename Op::Coef &K,
-                                           const typename Op::Extra &X, const BoundarySigns<typename Op::T> &sg) {
+                                           const char *B, int rank, int nl, int n, int iters, int first, int flip,
+                                           const typename Op::Coef &K, const typename Op::Extra &X,
+                                           const BoundarySigns<typename Op::T> &sg) {
   using T = typename Op::T;
   constexpr int E = (int)sizeof(T);
   const int us = L.us * E, bs = L.bs * E;
-  int xm[R][2], xp[R][2], ym[R][2], yp[R][2], zo[R][2], own[R];
-  unsigned left[R], right[R];
-  T v[R][2], b[R][2], d[R][2], rd[R][2], sxm[R], sxp[R], sym[R], syp[R], sz[R][2];
-#pragma unroll
-  for (int r = 0; r < R; r++) {
-    const int q = threadIdx.x + r * NT;
-    if (q >= n) continue;
-    const Pair p = make_pair_at<Op>(L, sg, smem_addr(U), rank, nl, q);
+  int a[6] = {}, ma[6] = {};  // x-, x+, y-, y+, outer z neighbour, own
+  T v = 0, w = 0, b = 0, d = 1, rd = 1, sxm = 1, sxp = 1, sym = 1, syp = 1, sz = 1;  // w: the pair's other cell
+  decltype(flip_bits(T(), T())) mb = 0, md = 0, mrd = 0, msz = 0;
+  unsigned left = 0, right = 0;
+  const bool mine = (int)threadIdx.x < n;
+  if (mine) {
+    const Pair p = make_pair_at<Op>(L, sg, smem_addr(U), rank, nl, threadIdx.x);
     const int c0 = (p.i + p.j) & 1;
-    own[r] = p.id;
-    left[r] = p.left;
-    right[r] = p.right;
-    sxm[r] = (p.self & 1) ? sg.xn : (T)1;
-    sxp[r] = (p.self & 2) ? sg.xp : (T)1;
-    sym[r] = (p.self & 4) ? sg.yn : (T)1;
-    syp[r] = (p.self & 8) ? sg.yp : (T)1;
+    left = p.left;
+    right = p.right;
+    if (SIGNED) {
+      sxm = (p.self & 1) ? sg.xn : (T)1;
+      sxp = (p.self & 2) ? sg.xp : (T)1;
+      sym = (p.self & 4) ? sg.yn : (T)1;
+      syp = (p.self & 8) ? sg.yp : (T)1;
+    }
 #pragma unroll
-    for (int c = 0; c < 2; c++) {
-      const bool odd = c != c0;
-      const int mine = c * us, other = (1 - c) * us;
-      v[r][c] = *reinterpret_cast<const T *>(U + mine + p.id);
-      b[r][c] = *reinterpret_cast<const T *>(B + c * bs + p.bid);
-      d[r][c] = cell_constant<Op>(P, L, K, p.i, p.j, 2 * p.m + odd, host);
-      rd[r][c] = Op::reciprocal(d[r][c]);
-      xm[r][c] = p.xm + ((p.self & 1) ? mine : other);
-      xp[r][c] = p.xp + ((p.self & 2) ? mine : other);
-      ym[r][c] = p.ym + ((p.self & 4) ? mine : other);
-      yp[r][c] = p.yp + ((p.self & 8) ? mine : other);
-      const bool face = p.self & (odd ? 32 : 16);
-      zo[r][c] = (odd ? p.zp : p.zm) + (face ? mine : other);
-      sz[r][c] = face ? (odd ? sg.zp : sg.zn) : (T)1;
+    for (int e = 1; e >= 0; e--) {  // e = 0: the cell of colour `first`
+      const int c = first ^ e, o = c * us, q = us - o;
+      const bool odd = c != c0, face = p.self & (odd ? 32 : 16);
+      const int t[6] = {p.xm + ((p.self & 1) ? o : q), p.xp + ((p.self & 2) ? o : q), p.ym + ((p.self & 4) ? o : q),
+                        p.yp + ((p.self & 8) ? o : q), (odd ? p.zp : p.zm) + (face ? o : q), p.id + o};
+#pragma unroll
+      for (int r = 0; r < 6; r++) {
+        ma[r] = a[r] ^ t[r];
+        a[r] = t[r];
+      }
+      w = v;
+      v = *reinterpret_cast<const T *>(U + o + p.id);
+      const T tb = *reinterpret_cast<const T *>(B + c * bs + p.bid);
+      const T td = cell_constant<Op>(P, L, K, p.i, p.j, 2 * p.m + odd, HOST), tr = Op::reciprocal(td);
+      const T ts = face ? (odd ? sg.zp : sg.zn) : (T)1;
+      mb = flip_bits(b, tb), md = flip_bits(d, td), mrd = flip_bits(rd, tr), msz = flip_bits(sz, ts);
+      b = tb, d = td, rd = tr, sz = ts;
     }
   }
-  auto at = [&](int off) { return *reinterpret_cast<const T *>(U + off); };
-  for (int it = 0; it < iters; it++) {
-    const int f = it < flip ? first : 1 - first;
+  int off = first * us;  // of the sweep's colour
+  auto at = [&](int o) { return *reinterpret_cast<const T *>(U + o); };
 #pragma unroll 1
-    for (int h = 0; h < 2; h++) {
-      auto phase = [&](auto colour) {
-        constexpr int c = decltype(colour)::value;
+  for (int ph = 0; ph < 2 * iters; ph++) {
+    if (ph != 0 && ph != 2 * flip) {  // the other colour, except where the order turns round
 #pragma unroll
-        for (int r = 0; r < R; r++) {
-          if ((int)threadIdx.x + r * NT < n) {
-            const T ax = at(xm[r][c]), bx = at(xp[r][c]), ay = at(ym[r][c]), by = at(yp[r][c]), az = at(zo[r][c]);
-            const T sx = SIGNED ? sxm[r] * ax + sxp[r] * bx : ax + bx;
-            const T sy = SIGNED ? sym[r] * ay + syp[r] * by : ay + by;
-            const T sz_ = (SIGNED ? sz[r][c] * az : az) + v[r][1 - c];
-            const T nv = Op::update(v[r][c], b[r][c], sx, sy, sz_, d[r][c], rd[r][c], K, X, host);
-            v[r][c] = nv;
-            *reinterpret_cast<T *>(U + c * us + own[r]) = nv;
-            st_cl_if(left[r], c * us, nv);
-            st_cl_if(right[r], c * us, nv);
-          }
-        }
-      };
-      if ((f ^ h) == 0) phase(std::integral_constant<int, 0>());
-      else phase(std::integral_constant<int, 1>());
-      level_barrier(L, l, nthreads);
+      for (int r = 0; r < 6; r++) a[r] ^= ma[r];
+      flip_value(b, mb);
+      flip_value(d, md);
+      if (Op::kHostCoarse) flip_value(rd, mrd);
+      if (SIGNED) flip_value(sz, msz);
+      const T o = v;
+      v = w;
+      w = o;
+      off = us - off;
     }
+    if (mine) {
+      const T ax = at(a[0]), bx = at(a[1]), ay = at(a[2]), by = at(a[3]), az = at(a[4]);
+      const T sx = SIGNED ? sxm * ax + sxp * bx : ax + bx;
+      const T sy = SIGNED ? sym * ay + syp * by : ay + by;
+      const T sz_ = (SIGNED ? sz * az : az) + w;
+      v = Op::update(v, b, sx, sy, sz_, d, rd, K, X, HOST);
+      *reinterpret_cast<T *>(U + a[5]) = v;
+      st_cl_if(left, off, v);
+      st_cl_if(right, off, v);
+    }
+    level_barrier(L, l, nthreads);
   }
 }
 
@@ -539,10 +552,12 @@ __device__ __forceinline__ void visit_level(const CtParams<Op> &P, int what, int
   if (iters > 0) {
     const bool plus = (sg.px || (sg.xn == (T)1 && sg.xp == (T)1)) && (sg.py || (sg.yn == (T)1 && sg.yp == (T)1)) &&
                       (sg.pz || (sg.zn == (T)1 && sg.zp == (T)1));
-    if (plus && most <= NT)
-      sweep_slab<Op, NT, 1, false>(P, L, l, nthreads, U, B, rank, nl, n, iters, first, flip, host, K, X, sg);
-    else if (most <= NT)
-      sweep_slab<Op, NT, 1, true>(P, L, l, nthreads, U, B, rank, nl, n, iters, first, flip, host, K, X, sg);
+    if (most <= NT && !host && plus) sweep_slab<Op, NT, false, false>(P, L, l, nthreads, U, B, rank, nl, n, iters, first, flip, K, X, sg);
+    else if (most <= NT && !host) sweep_slab<Op, NT, false, true>(P, L, l, nthreads, U, B, rank, nl, n, iters, first, flip, K, X, sg);
+    else if (Op::kHostCoarse && most <= NT && plus)
+      sweep_slab<Op, NT, Op::kHostCoarse, false>(P, L, l, nthreads, U, B, rank, nl, n, iters, first, flip, K, X, sg);
+    else if (Op::kHostCoarse && most <= NT)
+      sweep_slab<Op, NT, Op::kHostCoarse, true>(P, L, l, nthreads, U, B, rank, nl, n, iters, first, flip, K, X, sg);
     else {  // pairs worked out again in every phase
       for (int ph = 0; ph < 2 * iters; ph++) {
         const int color = (ph & 1) ^ (ph < 2 * flip ? first : 1 - first);

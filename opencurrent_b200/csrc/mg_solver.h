@@ -20,7 +20,8 @@ enum { RO_RED_BLACK = 0, RO_BLACK_RED = 1, RO_SYMMETRIC = 2 };
 
 int mg_num_levels(int nx, int ny, int nz);
 
-// The single-CTA coarse tail covers the 4^3 level only by default: measured at 256^3, a V-cycle
+// By default (tail_cells 0) the coarse levels run on one thread-block cluster (cluster_tail.cuh).  Where
+// the device cannot hold one, the single-CTA tail covers the 4^3 level only: measured at 256^3, a V-cycle
 // takes 0.558 ms (FP32) / 0.787 ms (FP64) with the tail at 64 cells against 0.581 / 0.810 ms at
 // 512 cells -- one SM runs a phase of an 8^3 level slower than a separate launch does.
 // (Ensembles run one tail CTA per member and use a larger tail.)
