@@ -162,8 +162,10 @@ typedef struct ocu_mg_params {
   int unfused;                   /* 1 = one launch per reference operation (no fused ghost
                                     writes, no fused residual+restriction, no tail kernel);
                                     same results, for A/B timing */
-  int tail_cells;                /* levels with at most this many cells run in one single-CTA
-                                    kernel per cycle; 0 = default (64), < 0 = off */
+  int tail_cells;                /* 0 (default) = the coarse levels run on one thread-block cluster
+                                    where the device can hold it; > 0 = levels with at most this
+                                    many cells run in one single-CTA kernel per cycle; < 0 = one
+                                    launch per operation down to the coarsest level */
   int sweep_cells;               /* levels with at least this many cells relax both colours in
                                     one TMA-fed pass (out of place, same results; Dirichlet and
                                     Neumann faces only); <= 0 = off (the default) */
