@@ -29,9 +29,7 @@
 #include <algorithm>
 #include <array>
 #include <atomic>
-#include <cstdlib>
 #include <cstring>
-#include <type_traits>
 #include <vector>
 
 #include "chq_device.cuh"
@@ -492,61 +490,61 @@ __device__ __forceinline__ void visit_level(const CtParams<Op> &P, int what, int
   hold(sg.xn), hold(sg.xp), hold(sg.yn), hold(sg.yp), hold(sg.zn), hold(sg.zp);
   auto at = [](const char *base, int off) { return *reinterpret_cast<const T *>(base + off); };
   if (what & CT_PROLONG) {
-      const LevelRegs Cl = level_regs(coarser);
-      for (int q = threadIdx.x; q < n; q += NT) {
-        const Pair p = make_pair_at<Op>(L, sg, ubase, rank, nl, q);
-        const int c0 = (p.i + p.j) & 1;
-        T v[2];
-        v[0] = at(U, c0 * us + p.id);
-        v[1] = at(U, (1 - c0) * us + p.id);
-        // prolongation: the four coarse rows of the pair's octant at K - 1, K, K + 1
-        const int I = p.i >> 1, J = p.j >> 1, Kz = p.m, M = Cl.M * E, S = Cl.ny * M, cus = Cl.us * E;
-        const bool xo = p.i & 1, yo = p.j & 1;
-        // x and y of the far rows and the sign of a value there (a face rule mirrors the row itself;
-        // periodic x neighbours are in the halo planes)
-        const bool fx = (xo ? I == Cl.nx - 1 : I == 0) && !sg.px, fy = yo ? J == Cl.ny - 1 : J == 0;
-        const int X1 = fx ? I : (xo ? I + 1 : I - 1);
-        const int Y1 = fy ? (sg.py ? (yo ? 0 : Cl.ny - 1) : J) : (yo ? J + 1 : J - 1);
-        const T s1 = fx ? (xo ? sg.xp : sg.xn) : (T)1, s2 = fy && !sg.py ? (yo ? sg.yp : sg.yn) : (T)1;
-        const bool bz = Kz == 0, tz = Kz == Cl.nz - 1;
-        const int Zm = bz ? (sg.pz ? Cl.nz - 1 : 0) : Kz - 1, Zp = tz ? (sg.pz ? 0 : Kz) : Kz + 1;
-        const T szm = bz && !sg.pz ? sg.zn : (T)1, szp = tz && !sg.pz ? sg.zp : (T)1;
-        const char *const cu = reinterpret_cast<const char *>(sm + Cl.ou) + (1 - (split_coarse ? rank * Cl.per : 0)) * S;
-        auto val = [&](int X, int Y, int Z) {
-          return at(cu, X * S + Y * M + (((X + Y + Z) & 1) ? cus : 0) + (Z >> 1) * E);
-        };
-        T c[4][3];  // rows (I, J), (X1, J), (I, Y1), (X1, Y1) at K, K - 1, K + 1
+    const LevelRegs Cl = level_regs(coarser);
+    for (int q = threadIdx.x; q < n; q += NT) {
+      const Pair p = make_pair_at<Op>(L, sg, ubase, rank, nl, q);
+      const int c0 = (p.i + p.j) & 1;
+      T v[2];
+      v[0] = at(U, c0 * us + p.id);
+      v[1] = at(U, (1 - c0) * us + p.id);
+      // prolongation: the four coarse rows of the pair's octant at K - 1, K, K + 1
+      const int I = p.i >> 1, J = p.j >> 1, Kz = p.m, M = Cl.M * E, S = Cl.ny * M, cus = Cl.us * E;
+      const bool xo = p.i & 1, yo = p.j & 1;
+      // x and y of the far rows and the sign of a value there (a face rule mirrors the row itself;
+      // periodic x neighbours are in the halo planes)
+      const bool fx = (xo ? I == Cl.nx - 1 : I == 0) && !sg.px, fy = yo ? J == Cl.ny - 1 : J == 0;
+      const int X1 = fx ? I : (xo ? I + 1 : I - 1);
+      const int Y1 = fy ? (sg.py ? (yo ? 0 : Cl.ny - 1) : J) : (yo ? J + 1 : J - 1);
+      const T s1 = fx ? (xo ? sg.xp : sg.xn) : (T)1, s2 = fy && !sg.py ? (yo ? sg.yp : sg.yn) : (T)1;
+      const bool bz = Kz == 0, tz = Kz == Cl.nz - 1;
+      const int Zm = bz ? (sg.pz ? Cl.nz - 1 : 0) : Kz - 1, Zp = tz ? (sg.pz ? 0 : Kz) : Kz + 1;
+      const T szm = bz && !sg.pz ? sg.zn : (T)1, szp = tz && !sg.pz ? sg.zp : (T)1;
+      const char *const cu = reinterpret_cast<const char *>(sm + Cl.ou) + (1 - (split_coarse ? rank * Cl.per : 0)) * S;
+      auto val = [&](int X, int Y, int Z) {
+        return at(cu, X * S + Y * M + (((X + Y + Z) & 1) ? cus : 0) + (Z >> 1) * E);
+      };
+      T c[4][3];  // rows (I, J), (X1, J), (I, Y1), (X1, Y1) at K, K - 1, K + 1
 #pragma unroll
-        for (int r = 0; r < 4; r++) {
-          const int X = (r & 1) ? X1 : I, Y = (r & 2) ? Y1 : J;
-          c[r][0] = val(X, Y, Kz);
-          c[r][1] = val(X, Y, Zm);
-          c[r][2] = val(X, Y, Zp);
-        }
-        T corner = 0;
-        if (Op::kCornerFromPlus) {
-          // the reference kernel takes the (-x, +y, +z) child's corner from coarse (+1, +1, +1)
-          const bool f2 = I == Cl.nx - 1 && !sg.px;
-          corner = (f2 ? sg.xp : (T)1) * (s2 * (szp * val(f2 ? I : I + 1, Y1, Zp)));
-        }
-#pragma unroll
-        for (int r = 0; r < 4; r++) {
-          const T s = ((r & 1) ? s1 : (T)1) * ((r & 2) ? s2 : (T)1);
-          c[r][0] = s * c[r][0];
-          c[r][1] = s * (szm * c[r][1]);
-          c[r][2] = s * (szp * c[r][2]);
-        }
-        if (!(Op::kCornerFromPlus && !xo && yo)) corner = c[3][2];
-        v[0] = Op::child(v[0], c[0][0], c[1][0], c[2][0], c[0][1], c[3][0], c[1][1], c[2][1], c[3][1]);
-        v[1] = Op::child(v[1], c[0][0], c[1][0], c[2][0], c[0][2], c[3][0], c[1][2], c[2][2], corner);
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const int o = (h ^ c0) * us;
-          *reinterpret_cast<T *>(U + o + p.id) = v[h];
-          st_cl_if(p.left, o, v[h]);
-          st_cl_if(p.right, o, v[h]);
-        }
+      for (int r = 0; r < 4; r++) {
+        const int X = (r & 1) ? X1 : I, Y = (r & 2) ? Y1 : J;
+        c[r][0] = val(X, Y, Kz);
+        c[r][1] = val(X, Y, Zm);
+        c[r][2] = val(X, Y, Zp);
       }
+      T corner = 0;
+      if (Op::kCornerFromPlus) {
+        // the reference kernel takes the (-x, +y, +z) child's corner from coarse (+1, +1, +1)
+        const bool f2 = I == Cl.nx - 1 && !sg.px;
+        corner = (f2 ? sg.xp : (T)1) * (s2 * (szp * val(f2 ? I : I + 1, Y1, Zp)));
+      }
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        const T s = ((r & 1) ? s1 : (T)1) * ((r & 2) ? s2 : (T)1);
+        c[r][0] = s * c[r][0];
+        c[r][1] = s * (szm * c[r][1]);
+        c[r][2] = s * (szp * c[r][2]);
+      }
+      if (!(Op::kCornerFromPlus && !xo && yo)) corner = c[3][2];
+      v[0] = Op::child(v[0], c[0][0], c[1][0], c[2][0], c[0][1], c[3][0], c[1][1], c[2][1], c[3][1]);
+      v[1] = Op::child(v[1], c[0][0], c[1][0], c[2][0], c[0][2], c[3][0], c[1][2], c[2][2], corner);
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int o = (h ^ c0) * us;
+        *reinterpret_cast<T *>(U + o + p.id) = v[h];
+        st_cl_if(p.left, o, v[h]);
+        st_cl_if(p.right, o, v[h]);
+      }
+    }
     level_barrier(L, l, nthreads);
   }
   if (iters > 0) {
@@ -584,35 +582,35 @@ __device__ __forceinline__ void visit_level(const CtParams<Op> &P, int what, int
   const LevelRegs Cl = level_regs(coarser);
   const int stride = Cl.per * Cl.ny * Cl.nz;  // residual scratch: elements per child
   {
-      for (int q = threadIdx.x; q < n; q += NT) {
-        const Pair p = make_pair_at<Op>(L, sg, ubase, rank, nl, q);
-        const int c0 = (p.i + p.j) & 1;
-        T b[2];
-        b[0] = at(B, c0 * bs + p.bid);
-        b[1] = at(B, (1 - c0) * bs + p.bid);
-        // residuals of both cells, stored into the scratch of the coarse cell's owner
-        const char *const Oe = U + (1 - c0) * us, *const Oo = U + c0 * us;  // other colour of the even / odd cell
-        const T e = at(U, c0 * us + p.id), o = at(U, (1 - c0) * us + p.id);
-        const T e0 = at(Oe, p.xm), e1 = at(Oe, p.xp), e2 = at(Oe, p.ym), e3 = at(Oe, p.yp), e4 = at(Oe, p.zm);
-        const T o0 = at(Oo, p.xm), o1 = at(Oo, p.xp), o2 = at(Oo, p.ym), o3 = at(Oo, p.yp), o5 = at(Oo, p.zp);
-        const T exs = ((p.self & 1) ? sg.xn * e : e0) + ((p.self & 2) ? sg.xp * e : e1);
-        const T oxs = ((p.self & 1) ? sg.xn * o : o0) + ((p.self & 2) ? sg.xp * o : o1);
-        const T eys = ((p.self & 4) ? sg.yn * e : e2) + ((p.self & 8) ? sg.yp * e : e3);
-        const T oys = ((p.self & 4) ? sg.yn * o : o2) + ((p.self & 8) ? sg.yp * o : o3);
-        const T ezs = ((p.self & 16) ? sg.zn * e : e4) + o;
-        const T ozs = e + ((p.self & 32) ? sg.zp * o : o5);
-        const int I = (p.i >> 1) - (split_coarse ? rank * Cl.per : 0);
-        const int to = P.orr + (4 * (p.i & 1) + 2 * (p.j & 1)) * stride + (I * Cl.ny + (p.j >> 1)) * Cl.nz + p.m;
-        const T re = Op::residual(e, b[0], exs, eys, ezs, K), ro = Op::residual(o, b[1], oxs, oys, ozs, K);
-        if (split_coarse == split_level) {  // this rank's own coarse cells
-          sm[to] = re;
-          sm[to + stride] = ro;
-        } else {
-          const unsigned far = map_rank(smem_addr(sm + to), 0);
-          st_cl(far, re);
-          st_cl(far + stride * E, ro);
-        }
+    for (int q = threadIdx.x; q < n; q += NT) {
+      const Pair p = make_pair_at<Op>(L, sg, ubase, rank, nl, q);
+      const int c0 = (p.i + p.j) & 1;
+      T b[2];
+      b[0] = at(B, c0 * bs + p.bid);
+      b[1] = at(B, (1 - c0) * bs + p.bid);
+      // residuals of both cells, stored into the scratch of the coarse cell's owner
+      const char *const Oe = U + (1 - c0) * us, *const Oo = U + c0 * us;  // other colour of the even / odd cell
+      const T e = at(U, c0 * us + p.id), o = at(U, (1 - c0) * us + p.id);
+      const T e0 = at(Oe, p.xm), e1 = at(Oe, p.xp), e2 = at(Oe, p.ym), e3 = at(Oe, p.yp), e4 = at(Oe, p.zm);
+      const T o0 = at(Oo, p.xm), o1 = at(Oo, p.xp), o2 = at(Oo, p.ym), o3 = at(Oo, p.yp), o5 = at(Oo, p.zp);
+      const T exs = ((p.self & 1) ? sg.xn * e : e0) + ((p.self & 2) ? sg.xp * e : e1);
+      const T oxs = ((p.self & 1) ? sg.xn * o : o0) + ((p.self & 2) ? sg.xp * o : o1);
+      const T eys = ((p.self & 4) ? sg.yn * e : e2) + ((p.self & 8) ? sg.yp * e : e3);
+      const T oys = ((p.self & 4) ? sg.yn * o : o2) + ((p.self & 8) ? sg.yp * o : o3);
+      const T ezs = ((p.self & 16) ? sg.zn * e : e4) + o;
+      const T ozs = e + ((p.self & 32) ? sg.zp * o : o5);
+      const int I = (p.i >> 1) - (split_coarse ? rank * Cl.per : 0);
+      const int to = P.orr + (4 * (p.i & 1) + 2 * (p.j & 1)) * stride + (I * Cl.ny + (p.j >> 1)) * Cl.nz + p.m;
+      const T re = Op::residual(e, b[0], exs, eys, ezs, K), ro = Op::residual(o, b[1], oxs, oys, ozs, K);
+      if (split_coarse == split_level) {  // this rank's own coarse cells
+        sm[to] = re;
+        sm[to + stride] = ro;
+      } else {
+        const unsigned far = map_rank(smem_addr(sm + to), 0);
+        st_cl(far, re);
+        st_cl(far + stride * E, ro);
       }
+    }
     // the residuals of a split level whose coarser level is split too are read by their own rank
     if (split_coarse) __syncthreads();
     else level_barrier(L, l, nthreads);
