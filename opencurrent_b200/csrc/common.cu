@@ -123,6 +123,13 @@ bool bc_any_periodic(const ocu_bc_set &s) {
          s.zpos.type == OCU_BC_PERIODIC || s.zneg.type == OCU_BC_PERIODIC;
 }
 
+bool bc_periodic_paired(const ocu_bc_set &s) {
+  const auto paired = [](const ocu_bc &a, const ocu_bc &b) {
+    return (a.type == OCU_BC_PERIODIC) == (b.type == OCU_BC_PERIODIC);
+  };
+  return paired(s.xpos, s.xneg) && paired(s.ypos, s.yneg) && paired(s.zpos, s.zneg);
+}
+
 // BoundaryConditionSet::make_homogeneous (ocuutil/boundary_condition.h:88-101)
 void bc_make_homogeneous(ocu_bc_set *s) {
   ocu_bc *f[6] = {&s->xpos, &s->xneg, &s->ypos, &s->yneg, &s->zpos, &s->zneg};

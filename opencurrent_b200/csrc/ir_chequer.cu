@@ -158,16 +158,13 @@ bool ChequerMG::suits(const std::vector<std::array<int, 3>> &dims, const ocu_bc_
   }
   // a periodic axis must be periodic on both faces and even on every level (the colouring
   // then continues across the wrap)
+  if (!bc_periodic_paired(bc)) return false;
   const bool per[3] = {bc.xpos.type == OCU_BC_PERIODIC, bc.ypos.type == OCU_BC_PERIODIC,
                        bc.zpos.type == OCU_BC_PERIODIC};
-  const bool per_neg[3] = {bc.xneg.type == OCU_BC_PERIODIC, bc.yneg.type == OCU_BC_PERIODIC,
-                           bc.zneg.type == OCU_BC_PERIODIC};
-  for (int a = 0; a < 3; a++) {
-    if (per[a] != per_neg[a]) return false;
+  for (int a = 0; a < 3; a++)
     if (per[a])
       for (const auto &d : dims)
         if (d[a] % 2) return false;
-  }
   for (const auto &d : dims)
     if ((long long)d[0] * d[1] * round4((d[2] + 1) / 2) / 4 >= (1LL << 31) / 8) return false;
   return level_smem(dims.back()) <= kTailSmemCap;

@@ -397,9 +397,11 @@ int MGCore<T>::tail_start() const {
 }
 
 // First level of the cluster's part, or -1 where the per-level kernels and the single-CTA tail run.
+// The cluster's levels wrap an axis or do not; an axis that is periodic on one face only keeps each
+// face's own rule, which the per-level kernels' ghost cells hold.
 template <typename T>
 int MGCore<T>::cluster_start() const {
-  return cluster && fused && !store_residuals ? cluster_tail_first<T>(dim) : -1;
+  return cluster && fused && !store_residuals && bc_periodic_paired(bc) ? cluster_tail_first<T>(dim) : -1;
 }
 
 template <typename T>

@@ -104,6 +104,8 @@ BCDev to_dev(const ocu_bc_set &bc);
 bool bc_check_scalar(const ocu_bc_set &bc);
 bool bc_check_mac(const ocu_bc_set &bc);
 bool bc_any_periodic(const ocu_bc_set &bc);
+// both faces of every axis agree on OCU_BC_PERIODIC (each face is accepted by itself elsewhere)
+bool bc_periodic_paired(const ocu_bc_set &bc);
 void bc_make_homogeneous(ocu_bc_set *bc);
 double bc_diag_mod(const ocu_bc &b, double factor);
 bool check_float(float f);

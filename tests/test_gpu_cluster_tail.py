@@ -5,6 +5,9 @@ import numpy as np
 import pytest
 
 import opencurrent_b200 as ocu
+from oracle import oracle_ctypes as O
+from tests.helpers import DIR as D, NEU as N, PER as P, bc_from, mg_params, npdt
+from tests.test_gpu_parity import assert_same, dev_grid, to_ocu_bc
 
 pytestmark = pytest.mark.gpu
 
@@ -67,3 +70,36 @@ def test_refinement_levels_bit_identical(dims, bc, monkeypatch):
         s.solve(1e-9, 3)
         got.append(s.pressure().copy_to_host())
     assert np.array_equal(*got, equal_nan=True)
+
+
+# An axis periodic on one face only: each face keeps its own rule on every level.
+ONE_SIDED = {f"{a}{per}_{'dirichlet' if other == D else 'neumann'}": (f"{a}{per}", f"{a}{'neg' if per == 'pos' else 'pos'}",
+                                                                       other)
+             for a in "xyz" for per in ("pos", "neg") for other in (D, N)}
+
+
+@pytest.mark.parametrize("dtype", [ocu.F32, ocu.F64])
+@pytest.mark.parametrize("name", list(ONE_SIDED))
+@pytest.mark.parametrize("rest", [N, P])
+def test_one_sided_periodic_axes(name, rest, dtype):
+    dims, h = (32, 24, 40), (0.03, 0.04, 0.03)
+    per, other, kind = ONE_SIDED[name]
+    faces = {f: (rest, 0.0) for f in ("xpos", "xneg", "ypos", "yneg", "zpos", "zneg")}
+    faces[per], faces[other] = (P, 0.0), (kind, 0.0)
+    bc = bc_from(faces)
+    L = O.layout(*dims)
+    rhs = np.zeros(int(L.allocated), npdt(dtype))
+    O.interior(rhs, L)[:] = np.random.default_rng(5).uniform(-1, 1, dims)
+    om = O.OracleMG("d" if dtype == ocu.F64 else "f", mg_params(bc), *dims, *h, rhs, L)
+    s = ocu.Sol_MultigridPressure3DDevice(dtype)
+    s.bc = to_ocu_bc(bc)
+    g = dev_grid(rhs, dtype, L)
+    s.initialize_storage(*dims, *h, g)
+    for one in (om, s):
+        one.run_fmg(1)
+        one.run_vcycles(2)
+    for l in range(om.num_levels):
+        for which, mine in (("u", s.read_u), ("b", s.read_b)):
+            want = om.grid(which, l)[0]
+            assert np.all(np.isfinite(want))
+            assert_same(mine(l).copy_to_host(), want, f"{which} of level {l}")
