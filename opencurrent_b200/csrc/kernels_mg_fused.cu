@@ -931,8 +931,11 @@ ocu_status launch_residual_restrict(const T *u, const T *b, const ocu_layout &Lf
                bc_, (int)Lc.xstride, (int)Lc.ystride, Lc.nx, Lc.ny, Lc.nz, zero_u, zero_n);
     return check_launch("k_residual_restrict_fine");
   }
+  // Two-wide loads where rows start on pairs and the buffers do: a caller's wrapped right-hand side
+  // need only have its element type's alignment.
   // (FP64 too: 256^3 solve 5759 -> 5692 us, 96x80x112 1930 -> 1898 against one load per operand)
-  if (Lf.shift % 2 == 0 && Lf.xstride % 2 == 0 && Lf.ystride % 2 == 0 && Lf.nz == 2 * Lc.nz) {
+  const bool pairs = ((reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(b)) & (2 * sizeof(T) - 1)) == 0;
+  if (pairs && Lf.shift % 2 == 0 && Lf.xstride % 2 == 0 && Lf.ystride % 2 == 0 && Lf.nz == 2 * Lc.nz) {
     if (rows2 || rowsinf) {
       launch_pdl(k_residual_restrict_v2<T, true>, grid, block, 0, s, u, b, Lf.xstride, Lf.ystride, Lf.nx, Lf.ny, Lf.nz,
                  c, bc_, Lc.xstride, Lc.ystride, Lc.nx, Lc.ny, Lc.nz, rows2, rowsinf, zero_u, zero_n);

@@ -167,3 +167,44 @@ def test_rayleigh_critical_number_on_gpu():
     from tests.rayleigh import critical_rayleigh_device
     ra = critical_rayleigh_device(16)
     assert abs(ra - 659.693989) < 3e-3, ra
+
+
+@pytest.mark.parametrize("norms", [False, True])
+def test_restriction_of_a_wrapped_rhs_with_element_alignment_only(norms):
+    """FP64 right-hand side in a caller's buffer that starts 8 bytes past a 16-byte boundary: the
+    residual + restriction reads it without pair loads, with the same result."""
+    import ctypes as C
+    import torch
+    dims, h = (48, 32, 40), (0.03, 0.03, 0.03)
+    L = O.layout(*dims)
+    host = np.random.default_rng(6).uniform(-1, 1, int(L.allocated))
+    flat = torch.zeros(int(L.allocated) + 2, dtype=torch.float64, device="cuda")
+    got = []
+    for offset in (0, 1):
+        t = flat[offset:offset + int(L.allocated)]
+        assert t.data_ptr() % 16 == 8 * offset
+        t.copy_(torch.from_numpy(host))
+        torch.cuda.synchronize()
+        handle = C.c_void_p()
+        ocu._capi.check(ocu.load().ocu_grid_wrap(F64, C.byref(dev_layout(L)), C.c_void_p(t.data_ptr()), C.byref(handle)))
+        g = ocu.Grid3DDevice(F64, _handle=handle.value)
+        g._owned = True
+        s = ocu.Sol_MultigridPressure3DDevice(F64)
+        s.bc = to_ocu_bc(bc_from(SCALAR_BCS["neumann"]))
+        s.convergence = ocu._capi.CONVERGENCE_NONE
+        s.initialize_storage(*dims, *h, g)
+        values = s.restrict_residuals(0, 1, norms=norms)
+        b1 = s.read_b(1).copy_to_host()
+        s.run_vcycles(2)
+        got.append((values, b1, s.pressure().copy_to_host()))
+        assert np.all(np.isfinite(got[-1][2]))
+    assert got[0][0] == got[1][0]
+    for a, b in zip(got[0][1:], got[1][1:]):
+        assert_same(a, b)
+
+
+def dev_layout(L):
+    d = ocu._capi.Layout()
+    for name, _ in d._fields_:
+        setattr(d, name, getattr(L, name))
+    return d
