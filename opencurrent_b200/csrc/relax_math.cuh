@@ -29,25 +29,26 @@ __device__ __forceinline__ T relax_res(T uc, T bv, T zm, T zp, T ym, T yp, T xm,
   return res;
 }
 
-// n / d, correctly rounded, for a divisor whose correctly rounded reciprocal r = 1 / d is at hand:
-// Markstein's theorem ("Computation of elementary functions on the IBM RISC System/6000
+// n / d, correctly rounded, for a positive divisor whose correctly rounded reciprocal r = 1 / d is at
+// hand: Markstein's theorem ("Computation of elementary functions on the IBM RISC System/6000
 // processor", 1990): q faithful to n / d and e = n - q d formed exactly give n / d correctly
 // rounded as q + e r.  The first correction makes the product n r faithful, the second is the
 // theorem's.  e is exact as long as nothing underflows, so numerators outside the guarded range
-// (zero apart, whose quotient every step keeps at zero) take the division itself.
-__device__ __forceinline__ float divide_by(float n, float d, float r) {
+// (zero apart) take the division itself.  Formed as -(q d - n), e is -0 for a zero numerator of
+// either sign, and q keeps its sign: with n - q d a -0 became +0.
+__host__ __device__ __forceinline__ float divide_by(float n, float d, float r) {
   const float m = fabsf(n);
   if ((m < 0x1p-90f && m > 0.f) || !(m < 0x1p90f)) return n / d;
   float q = n * r;
-  q = __fmaf_rn(__fmaf_rn(-q, d, n), r, q);
-  return __fmaf_rn(__fmaf_rn(-q, d, n), r, q);
+  q = fmaf(-fmaf(q, d, -n), r, q);
+  return fmaf(-fmaf(q, d, -n), r, q);
 }
-__device__ __forceinline__ double divide_by(double n, double d, double r) {
+__host__ __device__ __forceinline__ double divide_by(double n, double d, double r) {
   const double m = fabs(n);
   if ((m < 0x1p-800 && m > 0.0) || !(m < 0x1p800)) return n / d;
   double q = n * r;
-  q = __fma_rn(__fma_rn(-q, d, n), r, q);
-  return __fma_rn(__fma_rn(-q, d, n), r, q);
+  q = fma(-fma(q, d, -n), r, q);
+  return fma(-fma(q, d, -n), r, q);
 }
 
 // Diagonal of cell (i,j,k); away from every face it is c.ld exactly (nothing is added).
