@@ -5,10 +5,23 @@ namespace ocub {
 
 using namespace ct;
 
+// Most pairs of cells a rank may hold of a coarsest level that is relaxed by the level kernels'
+// arithmetic, one launch per colour otherwise.  A sweep costs the cluster one trip per kCtThreads pairs and
+// the launches nearly nothing more.  Four V-cycles of a two-level FP32 / FP64 hierarchy, launches -> cluster
+// (us): 30^3 (900 pairs) 6818 -> 4739 / 8311 -> 5800, 10x50x50 (1250) 19700 -> 16493 / 23058 -> 20532, but
+// 4x64x64 (2048) 30869 -> 35251 / 36848 -> 45002, 38^3 (2166) 11444 -> 14434 / 13810 -> 18063, 50^3 (5000)
+// 22280 -> 48234 / 27053 -> 62050.  The host routine's arithmetic is one CTA's work otherwise, and slower
+// there at every size (50^3: 1825 ms -> 51 ms).
+constexpr long long kCtDevicePairs = 3 * kCtThreads;
+
 template <typename T>
-int cluster_tail_first(const std::vector<std::array<int, 3>> &dims) {
+int cluster_tail_first(const std::vector<std::array<int, 3>> &dims, bool host_coarse) {
   const int ranks = ct_max_ranks<CtPlain<T>>();
-  return ranks ? ct_first<CtPlain<T>>(dims, 1, kCtTopCells, ranks) : -1;
+  if (!ranks) return -1;
+  const auto &d = dims.back();
+  const long long planes = (d[0] + ranks - 1) / ranks;
+  if (!host_coarse && planes * d[1] * (d[2] / 2) > kCtDevicePairs) return -1;
+  return ct_first<CtPlain<T>>(dims, 1, kCtTopCells, ranks);
 }
 
 template <typename T>
@@ -49,7 +62,7 @@ ocu_status launch_cluster_tail(const TailParams<T> &Q, bool ramp, cudaStream_t s
 }
 
 #define INST(T)                                                                     \
-  template int cluster_tail_first<T>(const std::vector<std::array<int, 3>> &);      \
+  template int cluster_tail_first<T>(const std::vector<std::array<int, 3>> &, bool); \
   template ocu_status launch_cluster_tail<T>(const TailParams<T> &, bool, cudaStream_t);
 INST(float)
 INST(double)

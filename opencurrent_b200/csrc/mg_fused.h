@@ -261,10 +261,11 @@ ocu_status launch_fold_rows(const T *rows, long long nrows, bool is_max, void *s
 template <typename T>
 ocu_status launch_coarse_tail(const TailParams<T> &P, cudaStream_t s);
 // The coarse end on one thread-block cluster (cluster_tail.cuh): the finest level >= 1 it takes,
-// or -1 (no level fits, or the device has no such clusters), and the launch of one V-cycle from
+// or -1 (no level fits, the device has no such clusters, or the coarsest level is faster as launches;
+// host_coarse: it is relaxed by the host routine's arithmetic), and the launch of one V-cycle from
 // lv[0], or of the FMG ramp up to and including lv[0]'s V-cycle (lv[0]'s u is then taken as zero).
 template <typename T>
-int cluster_tail_first(const std::vector<std::array<int, 3>> &dims);
+int cluster_tail_first(const std::vector<std::array<int, 3>> &dims, bool host_coarse);
 template <typename T>
 ocu_status launch_cluster_tail(const TailParams<T> &P, bool ramp, cudaStream_t s);
 // The single-CTA schedule for `members` grids at once, one CTA per member.

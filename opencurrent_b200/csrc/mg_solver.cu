@@ -401,7 +401,8 @@ int MGCore<T>::tail_start() const {
 // face's own rule, which the per-level kernels' ghost cells hold.
 template <typename T>
 int MGCore<T>::cluster_start() const {
-  return cluster && fused && !store_residuals && bc_periodic_paired(bc) ? cluster_tail_first<T>(dim) : -1;
+  return cluster && fused && !store_residuals && bc_periodic_paired(bc) ? cluster_tail_first<T>(dim, !disable_relax_on_host)
+                                                                        : -1;
 }
 
 template <typename T>

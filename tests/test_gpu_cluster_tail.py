@@ -103,3 +103,20 @@ def test_one_sided_periodic_axes(name, rest, dtype):
             want = om.grid(which, l)[0]
             assert np.all(np.isfinite(want))
             assert_same(mine(l).copy_to_host(), want, f"{which} of level {l}")
+
+
+@pytest.mark.parametrize("dtype", [ocu.F32, ocu.F64])
+@pytest.mark.parametrize("dims, clustered", [((60, 60, 60), True), ((20, 100, 100), True), ((8, 128, 128), False),
+                                             ((76, 76, 76), False)])
+def test_large_coarsest_level_stays_with_the_launches(dims, clustered, dtype):
+    """Relaxed by the level kernels' arithmetic, a coarsest level of more pairs than three trips of a
+    rank's threads is faster as launches: 900, 1250 pairs a rank below that line, 2048 and 2166 above."""
+    b = np.random.default_rng(7).uniform(-1, 1, dims)
+    counts = []
+    for knobs in (dict(), dict(tail_cells=-1)):
+        s = solver(ocu.Sol_MultigridPressure3DDevice(dtype), dims, BCS["dirichlet"], (b, dtype),
+                   disable_relax_on_host=True, **knobs)
+        n = ocu.kernel_launch_count()
+        s.run_vcycles(1)
+        counts.append(ocu.kernel_launch_count() - n)
+    assert (counts[0] < counts[1]) if clustered else (counts[0] == counts[1])
