@@ -869,6 +869,9 @@ inline int ct_max_ranks() {
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   std::atomic<int> &k = known[dev & 63];
   if (k.load() == 0) {
+    // An error that an earlier call left is for the next launch to report: the questions below would
+    // clear it (cudaFuncSetAttribute does), so they are left for another time.
+    if (cudaPeekAtLastError() != cudaSuccess) return 0;
     int found = -1;
     bool ok = true;
     const void *f = (const void *)k_cluster_tail<Op, kCtThreads>;

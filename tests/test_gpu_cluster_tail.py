@@ -1,6 +1,10 @@
 """The coarse levels on one thread-block cluster against the per-level kernels: every level's u and b
 (ghosts included) bit for bit after a fixed schedule, and the refinement solver's pressure against
 its single-CTA tail's."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -120,3 +124,35 @@ def test_large_coarsest_level_stays_with_the_launches(dims, clustered, dtype):
         s.run_vcycles(1)
         counts.append(ocu.kernel_launch_count() - n)
     assert (counts[0] < counts[1]) if clustered else (counts[0] == counts[1])
+
+
+EARLIER_ERROR = """
+import opencurrent_b200 as ocu
+from opencurrent_b200._capi import ERR_ALLOC, ERR_CUDA
+for attempt in range(2):  # the device is asked for its cluster size in the first solve only
+    rhs = ocu.Grid3DDevice(ocu.F32)
+    rhs.init(32, 32, 32)
+    s = ocu.Sol_MultigridPressure3DDevice(ocu.F32)
+    s.bc = ocu.BoundaryConditionSet(ocu.BoundaryCondition(ocu.BC_NEUMANN))
+    s.initialize_storage(32, 32, 32, 1 / 32, 1 / 32, 1 / 32, rhs)
+    try:
+        ocu.Grid3DDevice(ocu.F32).init(20000, 20000, 20000)  # 32 TB
+        raise SystemExit("allocated")
+    except ocu.OcuError as e:
+        assert e.status == ERR_ALLOC, e
+    try:
+        s.run_vcycles(1)
+        print("taken")
+    except ocu.OcuError as e:
+        assert e.status == ERR_CUDA and "out of memory" in str(e), e
+        print("reported")
+    s.run_vcycles(1)
+"""
+
+
+def test_asking_for_the_cluster_size_keeps_an_earlier_error():
+    """A refused allocation leaves its error with the thread, and the next launch reports it, in a
+    program's first solve as in any other."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", EARLIER_ERROR], capture_output=True, text=True, timeout=300, cwd=root)
+    assert r.returncode == 0 and r.stdout.split() == ["reported", "reported"], r.stdout + r.stderr
