@@ -1,6 +1,6 @@
 """The coarse levels on one thread-block cluster against the per-level kernels: every level's u and b
 (ghosts included) bit for bit after a fixed schedule, and the refinement solver's pressure against
-its single-CTA tail's."""
+its single-CTA tail's; which hierarchies the cluster takes, by their launch counts."""
 import os
 import subprocess
 import sys
@@ -22,8 +22,9 @@ BCS = {"neumann": ocu.BoundaryConditionSet(NEU), "dirichlet": ocu.BoundaryCondit
        "mixed": ocu.BoundaryConditionSet(NEU, xpos=PER, xneg=PER, zpos=DIR),
        "open": ocu.BoundaryConditionSet(DIR, ypos=NONE, zneg=NEU)}
 # coarse levels held by one CTA only; split over few and over all 16 ranks; uneven planes per rank; a
-# coarsest level with more than one pair per thread; two planes along x
+# coarsest level (4x32x48, four ranks of one plane) with more than one pair per thread
 SHAPES = [(16, 16, 16), (64, 64, 64), (40, 24, 56), (96, 80, 48), (72, 64, 36), (68, 16, 20), (8, 64, 96)]
+SYMMETRIC = [(40, 24, 56), (72, 64, 36)]
 
 
 def solver(cls, dims, bc, b, **knobs):
@@ -44,36 +45,52 @@ def solver(cls, dims, bc, b, **knobs):
     return s
 
 
+def bits(a):
+    return a.view(np.int64 if a.dtype == np.float64 else np.int32)
+
+
+def launches(f):
+    n = ocu.kernel_launch_count()
+    f()
+    return ocu.kernel_launch_count() - n
+
+
 @pytest.mark.parametrize("dtype", [ocu.F32, ocu.F64])
 @pytest.mark.parametrize("bc", list(BCS))
 @pytest.mark.parametrize("dims", SHAPES)
-def test_levels_bit_identical(dims, bc, dtype):
+@pytest.mark.parametrize("level_arithmetic", [False, True])  # of the coarsest level: the host routine's or the others'
+def test_levels_bit_identical(level_arithmetic, dims, bc, dtype):
     b = np.random.default_rng(3).uniform(-1, 1, dims)
-    sym = dims == (40, 24, 56)
-    got = []
+    got, counts = [], []
     for knobs in (dict(), dict(tail_cells=-1)):
-        s = solver(ocu.Sol_MultigridPressure3DDevice(dtype), dims, BCS[bc], (b, dtype), make_symmetric_operator=sym,
-                   disable_relax_on_host=dims == (96, 80, 48), nu2=1 if dims == (64, 64, 64) else 2, **knobs)
-        s.run_fmg(1)
-        s.run_vcycles(2)
+        s = solver(ocu.Sol_MultigridPressure3DDevice(dtype), dims, BCS[bc], (b, dtype),
+                   make_symmetric_operator=dims in SYMMETRIC, disable_relax_on_host=level_arithmetic,
+                   nu2=1 if dims == (64, 64, 64) else 2, **knobs)
+        counts.append(launches(lambda: (s.run_fmg(1), s.run_vcycles(2))))
         got.append([g(l).copy_to_host() for l in range(s.stats.num_levels) for g in (s.read_u, s.read_b)])
+    # the cluster took its levels (a coarsest level alone is one launch by the host routine's arithmetic too)
+    assert counts[0] < counts[1] or (s.stats.num_levels == 2 and not level_arithmetic)
     for one, other in zip(*got):
-        assert np.array_equal(one, other, equal_nan=True)
+        assert np.all(np.isfinite(other))
+        assert np.array_equal(bits(one), bits(other))
 
 
-@pytest.mark.parametrize("dims", SHAPES)
+# (8, 8, 8): the whole hierarchy in the tail, its ramp ending with level 0's own V-cycle
+@pytest.mark.parametrize("dims", SHAPES + [(8, 8, 8)])
 @pytest.mark.parametrize("bc", ["neumann", "mixed", "periodic"])
 def test_refinement_levels_bit_identical(dims, bc, monkeypatch):
     b = np.random.default_rng(4).uniform(-1, 1, dims)
     b -= b.mean()
-    got = []
+    got, counts = [], []
     for env in (None, "512"):
         if env:
             monkeypatch.setenv("OCU_B200_CHQ_TAIL", env)
         s = solver(ocu.Sol_MultigridPressureMixed3DDeviceD(), dims, BCS[bc], (b, ocu.F64))
-        s.solve(1e-9, 3)
+        counts.append(launches(lambda: s.solve(1e-9, 3)))
         got.append(s.pressure().copy_to_host())
-    assert np.array_equal(*got, equal_nan=True)
+    assert counts[0] < counts[1] or s.stats.num_levels == 2  # two levels: the coarsest is one launch either way
+    assert np.all(np.isfinite(got[1]))
+    assert np.array_equal(*map(bits, got))
 
 
 # An axis periodic on one face only: each face keeps its own rule on every level.
@@ -120,9 +137,7 @@ def test_large_coarsest_level_stays_with_the_launches(dims, clustered, dtype):
     for knobs in (dict(), dict(tail_cells=-1)):
         s = solver(ocu.Sol_MultigridPressure3DDevice(dtype), dims, BCS["dirichlet"], (b, dtype),
                    disable_relax_on_host=True, **knobs)
-        n = ocu.kernel_launch_count()
-        s.run_vcycles(1)
-        counts.append(ocu.kernel_launch_count() - n)
+        counts.append(launches(lambda: s.run_vcycles(1)))
     assert (counts[0] < counts[1]) if clustered else (counts[0] == counts[1])
 
 
