@@ -805,9 +805,32 @@ def run_kernel_case(args):
         s.prolong(1, 0, core=2)
         s.synchronize()
         rms = float(np.sqrt(np.mean(fourier_rhs(n) ** 2)))
-        s.solve(1e-10 * rms, 30)   # one whole solve: its coarse end runs the single-CTA kernel
+        s.solve(1e-10 * rms, 30)   # one whole solve: its coarse end runs k_cluster_tail
         torch.cuda.synchronize()
         print(json.dumps({"kernel_case": "chequer", "grid": [n] * 3, "ok": True}), flush=True)
+        return
+
+    if args.kernel_case == "cluster":
+        # k_cluster_tail alone is of interest: per configuration two V-cycles, two launches of it.
+        # More iterations on the levels above the coarsest (nu) tell a sweep's cost from the rest.
+        cases = [(dt, dims, nu) for dims in ((16, 16, 16), (32, 32, 32), (64, 64, 32)) for dt in ("f32", "f64") for nu in (2, 6)]
+        cases += [("f64", (24, 20, 28), 2), ("f32", (48, 40, 36), 2)]  # coarsest 12x10x14 and 24x20x18
+        keep = []
+        for dt, dims, nu in cases:
+            dtype = ocu.F64 if dt == "f64" else ocu.F32
+            rhs = ocu.Grid3DDevice(dtype)
+            rhs.init(*dims)
+            b = np.random.default_rng(0).uniform(-1.0, 1.0, dims)
+            rhs.copy_from_host(padded(b - b.mean(), ocu.layout(*dims), np.float64 if dt == "f64" else np.float32))
+            s = ocu.Sol_MultigridPressure3DDevice(dtype)
+            s.bc = ocu.BoundaryConditionSet(ocu.BoundaryCondition(ocu.BC_NEUMANN, 0.0))
+            s.nu1 = s.nu2 = nu
+            s.initialize_storage(*dims, *(1.0 / max(dims),) * 3, rhs)
+            s.run_vcycles(2)
+            keep.append((rhs, s))
+        torch.cuda.synchronize()
+        print(json.dumps({"kernel_case": "cluster", "two_launches_each": [f"{dt} {d} nu {nu}" for dt, d, nu in cases],
+                          "ok": True}), flush=True)
         return
 
     if args.kernel_case == "flow":
@@ -838,7 +861,7 @@ def run_kernel_case(args):
     elif args.kernel_case == "restrict":
         s.restrict_residuals(0, 1, norms=True)
     elif args.kernel_case == "tail":
-        s.run_vcycles(1)          # one V-cycle: its coarse end is one k_coarse_tail_smem launch
+        s.run_vcycles(1)          # one V-cycle: its coarse end is one k_cluster_tail launch
     s.synchronize()
     torch.cuda.synchronize()
     print(json.dumps({"kernel_case": args.kernel_case, "grid": [n] * 3, "ok": True}), flush=True)
@@ -855,9 +878,9 @@ def main():
                     help="levels with at least this many cells use the two-colour TMA pass (0 = off)")
     ap.add_argument("--skip-cpu", action="store_true")
     ap.add_argument("--skip-secondary", action="store_true")
-    ap.add_argument("--kernel-case", choices=["relax", "prolong", "restrict", "tail", "flow", "chequer"],
-                    help="run a few launches of one kernel on the 256^3 FP32 hierarchy, or two "
-                         "256x256x128 flow steps (profiling)")
+    ap.add_argument("--kernel-case", choices=["relax", "prolong", "restrict", "tail", "flow", "chequer", "cluster"],
+                    help="run a few launches of one kernel on the 256^3 FP32 hierarchy, two "
+                         "256x256x128 flow steps, or the coarse end of small hierarchies (profiling)")
     args = ap.parse_args()
     if args.kernel_case:
         run_kernel_case(args)

@@ -35,7 +35,7 @@ ocu_status launch_cluster_tail(const TailParams<T> &Q, bool ramp, cudaStream_t s
   for (int l = 0; l < Q.nlev; l++) {
     const TailLevel<T> &v = Q.lv[l];
     P.lv[l].k = {v.rc, v.res};
-    P.lv[l].g = {v.u, v.b, v.xs, v.ys, v.hx, v.hy, v.hz};
+    P.lv[l].g = {v.u, v.b, v.xs, v.ys};
   }
   P.nu1 = Q.nu1;
   P.nu2 = Q.nu2;
@@ -50,13 +50,7 @@ ocu_status launch_cluster_tail(const TailParams<T> &Q, bool ramp, cudaStream_t s
   P.x.cc = Q.cc;
   P.x.unit = Q.cc.fx == 1 && Q.cc.fy == 1 && Q.cc.fz == 1;
   P.x.bc = Q.lv[0].bc;
-  auto sign = [&](int f) {
-    const int t = P.x.bc.type[f];
-    return (T)(t == OCU_BC_NEUMANN ? 1 : t == OCU_BC_DIRICHELET ? -1 : 0);
-  };
-  auto periodic = [&](int f) { return P.x.bc.type[f] == OCU_BC_PERIODIC ? 1 : 0; };
-  P.sg = {sign(FX_NEG), sign(FX_POS), sign(FY_NEG), sign(FY_POS), sign(FZ_NEG), sign(FZ_POS),
-          periodic(FX_POS), periodic(FY_POS), periodic(FZ_POS)};
+  P.sg = boundary_signs<T>(P.x.bc);
   ct_schedule(P, ramp, ramp ? 0 : 1, Q.first_level == 0, 1LL << 62);
   return ct_launch(P, ranks, bytes, s);
 }

@@ -5,9 +5,11 @@
 //
 // What bounds it: a phase over such a level is a chain of shared-memory loads, one SOR update
 // and a barrier; no unit is near its throughput.  A launch with programmatic dependencies costs
-// 2.2-2.5 us whatever the level's size; a cluster phase costs 0.45-0.6 us (a barrier over 16 CTAs
-// of 512 threads 0.24 us, over one CTA 0.23 us, measured).  One CTA alone is the cheaper home
-// only where its threads hold the level in one or two trips (kCtSingleCells).
+// 2.2-2.5 us whatever the level's size; a colour sweep here 0.25 us (FP64 0.33) on an 8^3 level held
+// by one CTA, 0.45 (0.5) on a 16^3 level over 16 and 0.55 on a 24x20x18 one over 12
+// (bench.py --kernel-case cluster under ncu), of which a barrier alone is 0.24 us over 16 CTAs of 512 threads and
+// 0.22 over one.  One CTA alone is the cheaper home only where its threads hold the level in one or
+// two trips (kCtSingleCells).  Cycle counts in this file are clock64 differences inside the kernel.
 //
 // Layout.  As the split levels of ir_chequer.h: per colour c (cell (i,j,k) has colour (i+j+k)&1)
 // one array of rows (i,j), cell k at entry m = k >> 1 -- all sizes of a level are even, since a
@@ -55,14 +57,15 @@ template <typename T> struct BoundarySigns {
   int px, py, pz;
 };
 
-inline double sign_of(const ocu_bc &b) {
-  return b.type == OCU_BC_NEUMANN ? 1.0 : b.type == OCU_BC_DIRICHELET ? -1.0 : 0.0;
-}
+// (an axis wraps at both ends or at neither: bc_periodic_paired)
 template <typename T>
-inline BoundarySigns<T> boundary_signs(const ocu_bc_set &b) {
-  return {(T)sign_of(b.xneg), (T)sign_of(b.xpos), (T)sign_of(b.yneg), (T)sign_of(b.ypos),
-          (T)sign_of(b.zneg), (T)sign_of(b.zpos), b.xpos.type == OCU_BC_PERIODIC,
-          b.ypos.type == OCU_BC_PERIODIC, b.zpos.type == OCU_BC_PERIODIC};
+inline BoundarySigns<T> boundary_signs(const BCDev &b) {
+  auto sign = [&](int f) {
+    return (T)(b.type[f] == OCU_BC_NEUMANN ? 1 : b.type[f] == OCU_BC_DIRICHELET ? -1 : 0);
+  };
+  auto wraps = [&](int f) { return b.type[f] == OCU_BC_PERIODIC ? 1 : 0; };
+  return {sign(FX_NEG), sign(FX_POS), sign(FY_NEG), sign(FY_POS), sign(FZ_NEG), sign(FZ_POS),
+          wraps(FX_POS), wraps(FY_POS), wraps(FZ_POS)};
 }
 
 // Keeps a value in a register: the level records are indexed at run time, and the compiler would
@@ -89,7 +92,6 @@ struct CtPlain {
   struct Global {
     T *u, *b;
     long long xs, ys;
-    T hx, hy, hz;
   };
   static constexpr bool kHostCoarse = true;
   static __device__ __forceinline__ void hold(Coef &c) {
@@ -107,9 +109,9 @@ struct CtPlain {
     const T zm = (k == 0) ? c.zn : (k == nz - 1) ? c.zp : (T)0;
     return c.ld + xm + ym + zm;
   }
-  // host: the coarsest level's arithmetic
   // the update's division: by the cell's diagonal, whose reciprocal is worked out once
   static __device__ __forceinline__ T reciprocal(T dg) { return (T)1 / dg; }
+  // host: the coarsest level's arithmetic
   static __device__ __forceinline__ T update(T u, T b, T sx, T sy, T sz, T dg, T rdg, const Coef &c, const Extra &x,
                                              bool host) {
     const CoarseCoef<T> &h = x.cc;

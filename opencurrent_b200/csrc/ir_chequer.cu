@@ -280,7 +280,7 @@ ocu_status ChequerMG::tail_cluster(bool fmg, int more, int nu1, int nu2, int cit
   P.nu1 = nu1;
   P.nu2 = nu2;
   P.coarse_iters = P.coarse_flip = citers;
-  P.sg = ct::boundary_signs<float>(bc);
+  P.sg = ct::boundary_signs<float>(to_dev(bc));
   const ChqBC b = make_bc(bc, fx, fy, fz);
   P.x = {b.mxn, b.mxp, b.myn, b.myp, b.mzn, b.mzp};
   P.ramp_iters = ramp_iters;

@@ -381,8 +381,9 @@ ocu_status MGCore<T>::prolong(int coarse, int fine) {
   return apply_bc(fine);
 }
 
-// First level handled by the single-CTA tail: the finest level >= 1 from which every level has
-// at most tail_cells cells.  num_levels-1 means "coarsest only" (the plain coarse kernel).
+// First level of the part that runs as one launch: the cluster's where it takes any, else the
+// single-CTA tail's, the finest level >= 1 from which every level has at most tail_cells cells.
+// num_levels-1 in that case means "coarsest only" (the plain coarse kernel).
 template <typename T>
 int MGCore<T>::tail_start() const {
   const int coarse = num_levels - 1;
@@ -525,14 +526,14 @@ static double pick(int conv, double l2, double linf) {
 // CUDA-graph replay.  The schedule between two host decisions is fixed for a given solver
 // configuration, so each such segment is captured once (stream capture of the same enqueue
 // code) and replayed with one cudaGraphLaunch:
-//   INIT   ghost fill of u0 + residual norms of level 0 (read back, then decide)
-//   RAMP   restriction chain + the FMG cycles from the coarsest level up to level 1
-//   PRE0   pre-smooth at level 0, clear level 1, residual+restriction+norms (read back)
-//   REST0  the rest of a level-0 cycle (levels 1.. down, tail kernel, up to level 0)
-// What runs between two readbacks is one graph (the ramp with the first PRE0, a REST0 with the next
-// cycle's PRE0), so that the programmatic dependencies are not broken between them; a REST0 on its
-// own ends a run that stops at max_iter.
-//   FINAL  ghost fill of u0 after convergence
+//   INIT        ghost fill of u0 + residual norms of level 0 (read back, then decide)
+//   RAMP_PRE0   restriction chain + the FMG cycles from the coarsest level up to level 1, then
+//   PRE0        pre-smooth at level 0, clear level 1, residual+restriction+norms (read back)
+//   REST0_PRE0  the rest of a level-0 cycle (levels 1.. down, the tail, up to level 0), then PRE0
+//   REST0       the rest of the last cycle of a run that stops at max_iter
+//   FINAL       ghost fill of u0 after convergence
+// PRE0 has a graph of its own where a V-cycle run begins.  What runs between two readbacks is one
+// graph, so that the programmatic dependencies are not broken between its parts.
 // With CONVERGENCE_NONE nothing is read back, so a whole fixed-schedule FMG (the refinement
 // solver's inner solve) runs as a chain of graph launches without a host wait.
 // ------------------------------------------------------------------------------------------
@@ -745,7 +746,7 @@ ocu_status MGSolver::do_fmg(double tolerance, int max_iter, double *rl2, double 
 }
 
 // One V-cycle from fine_level (the body of the cycle loops of do_fmg and do_vcycle).  The
-// levels from tail_start() down are handed to the single-CTA tail kernel; at level 0 the
+// levels from tail_start() down are handed to the tail (cycle_tail); at level 0 the
 // residual norm is read back after the pre-smooth and the cycle stops when it is below the
 // tolerance, after refreshing the level-0 ghosts (sol_mgpressure3d.cpp:186-236).
 ocu_status MGSolver::cycle(CoreOps *c, int fine_level, double tolerance, double *rl2, double *rlinf,
