@@ -163,7 +163,9 @@ typedef struct ocu_mg_params {
                                     writes, no fused residual+restriction, no tail kernel);
                                     same results, for A/B timing */
   int tail_cells;                /* 0 (default) = the coarse levels run on one thread-block cluster
-                                    where the device can hold it; > 0 = levels with at most this
+                                    where the device can hold it, no axis is periodic on one face
+                                    only, and the coarsest level is not large and relaxed by the
+                                    level kernels' arithmetic; > 0 = levels with at most this
                                     many cells run in one single-CTA kernel per cycle; < 0 = one
                                     launch per operation down to the coarsest level */
   int sweep_cells;               /* levels with at least this many cells relax both colours in
